@@ -441,6 +441,12 @@ int mgd_profile_stage_kernels(mgd_ctx* ctx, int mode, int reps, double* avg_ms, 
  * CUDA's pow (ref), for checking the viscosity law's error bound. */
 int mgd_selftest_pow(const double* x, int n, double e, double* fast, double* ref);
 
+/* Self-test of the interior stencils, which run in integer arithmetic: x
+   holds n windows of nine taps (offsets -4..4), out the n results of op 0
+   (first derivative), 1 (its adjoint) or 2 (composite dissipation) of the
+   MGD_SBP_* scheme. */
+int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out);
+
 /* Self-test of the bounded wait of the persistent batched kernel (no
  * reference counterpart), used as a grid barrier: a cooperative launch of
  * n_blocks CTAs meets `rounds` times at a barrier that expects `expected`

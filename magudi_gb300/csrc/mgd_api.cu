@@ -3298,6 +3298,22 @@ int mgd_selftest_fp64_rate(int warps_per_sm, double* lane_ops_per_clock) {
 
 // Self-test of the table-driven power function used by the viscosity law:
 // evaluates x[i]^e with it (fast) and with CUDA's pow (ref) on the current device.
+int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out) {
+  if (!x || !out || n < 1 || n > (1 << 24) || scheme < 0 || scheme >= kSchemes || op < 0 || op > 2) return 1;
+  double *dx = nullptr, *dout = nullptr;
+  cudaError_t e = cudaMalloc((void**)&dx, (size_t)n * 9 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&dout, (size_t)n * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemcpy(dx, x, (size_t)n * 9 * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    launchStencilSelfTest(dx, n, scheme, op, dout);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(out, dout, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost);
+  cudaFree(dx);
+  cudaFree(dout);
+  return e == cudaSuccess ? 0 : 1;
+}
+
 int mgd_selftest_pow(const double* x, int n, double e, double* fast, double* ref) {
   if (n <= 0) return 0;
   double *dx = nullptr, *df = nullptr, *dr = nullptr;

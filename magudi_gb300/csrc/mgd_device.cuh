@@ -10,6 +10,8 @@
 
 #include <cstdint>
 
+#include "mgd_fixed.cuh"
+
 namespace mgd {
 
 enum OpId { OP_D1 = 0, OP_D1ADJ = 1, OP_DISS = 2, OP_DISST = 3, OP_DCOMP = 4, OP_COUNT = 5 };
@@ -31,6 +33,7 @@ constexpr int kSchemes = 4;
 struct OpTables {
   double interior[kSchemes][OP_COUNT][9];  // offsets -half..half
   int asym[kSchemes][OP_COUNT];            // general interior sum and explicit right block
+  FixedOp fixed[kSchemes][OP_COUNT];       // integer interiors (OP_D1, OP_D1ADJ, OP_DCOMP)
 };
 
 // One copy per translation unit; only mgd_kernels.cu launches kernels and
@@ -75,78 +78,136 @@ __device__ __forceinline__ double tap(const double* p) {
   else return __ldca(p);
 }
 
-template <int OP, bool NC = true, int CU = 1>
-__device__ __forceinline__ double applyOp(const double* __restrict__ line, int i, const Axis& ax) {
+// Interior stencil of OP over the taps p[j] = x_{j+1}, m[j] = x_{-(j+1)} and
+// the centre x0 (unused by skew operators): the first derivatives in integers
+// where the taps allow it, else in FP64, left to right.
+template <int OP>
+__device__ __forceinline__ double interiorSum(const double* p, const double* m, double x0, int scheme) {
   using S = OpShape<OP>;
-  const double* __restrict__ cin = c_ops.interior[ax.scheme][OP];
+  if constexpr (OP == OP_D1 || OP == OP_D1ADJ) {
+    double s;
+    if (c_ops.fixed[scheme][OP].valid && fixedSkew(p, m, c_ops.fixed[scheme][OP], s)) return s;
+  }
+  const double* __restrict__ cin = c_ops.interior[scheme][OP];
+  double s = cin[S::half + 1] * (S::skew ? p[0] - m[0] : p[0] + m[0]);
+#pragma unroll
+  for (int j = 2; j <= S::half; ++j) s += cin[S::half + j] * (S::skew ? p[j - 1] - m[j - 1] : p[j - 1] + m[j - 1]);
+  return S::skew ? s : s + cin[S::half] * x0;
+}
+
+// Boundary closure row of point i (i < depth or i >= n - depth) of a
+// non-periodic line: CU taps' loads in flight at a time; the sum keeps its
+// order either way. c points at the line's point i.
+template <int OP, bool NC, int CU>
+__device__ __forceinline__ double closureSum(const double* __restrict__ c, int i, long long st, const Axis& ax) {
+  using S = OpShape<OP>;
+  const double* __restrict__ line = c - i * st;
+  if (i < S::depth) {
+    const double* __restrict__ row = &g_opLeft[ax.scheme][OP][i * S::width];
+    double s = __ldg(row) * tap<NC>(line);
+#pragma unroll CU
+    for (int k = 1; k < S::width; ++k) s += __ldg(row + k) * tap<NC>(line + k * st);
+    return s;
+  }
+  const int m = ax.n - 1 - i;
+  const double* __restrict__ end = line + (long long)(ax.n - S::width) * st;
   // only the non-composite dissipation pair of SBP 3-6 is asymmetric
-  const bool asym = !S::skew && (OP == OP_DISS || OP == OP_DISST) && c_ops.asym[ax.scheme][OP];
-  const long long st = ax.stride;
-  if (ax.per == 0) {
-    if (i < S::depth) {
-      // boundary closure rows: CU taps' loads in flight at a time (the sum
-      // keeps its order either way)
-      const double* __restrict__ row = &g_opLeft[ax.scheme][OP][i * S::width];
-      double s = __ldg(row) * tap<NC>(line);
+  if (!S::skew && (OP == OP_DISS || OP == OP_DISST) && c_ops.asym[ax.scheme][OP]) {
+    // explicit right block, columns left to right
+    const double* __restrict__ row = &g_opRight[ax.scheme][OP][m * S::width];
+    double s = __ldg(row) * tap<NC>(end);
 #pragma unroll CU
-      for (int k = 1; k < S::width; ++k) s += __ldg(row + k) * tap<NC>(line + k * st);
-      return s;
-    }
-    if (i >= ax.n - S::depth) {
-      const int m = ax.n - 1 - i;
-      const double* __restrict__ end = line + (long long)(ax.n - S::width) * st;
-      if (asym) {
-        // explicit right block, columns left to right
-        const double* __restrict__ row = &g_opRight[ax.scheme][OP][m * S::width];
-        double s = __ldg(row) * tap<NC>(end);
-#pragma unroll CU
-        for (int k = 1; k < S::width; ++k) s += __ldg(row + k) * tap<NC>(end + k * st);
-        return s;
-      }
-      const double* __restrict__ row = &g_opLeft[ax.scheme][OP][m * S::width];
-      // right block = reflection of the left block, negated for skew operators
-      double s = __ldg(row + S::width - 1) * tap<NC>(end);
-#pragma unroll CU
-      for (int k = 1; k < S::width; ++k) s += __ldg(row + S::width - 1 - k) * tap<NC>(end + k * st);
-      return S::skew ? -s : s;
-    }
-    const double* __restrict__ c = line + (long long)i * st;
-    if (S::skew) {
-      double s = cin[S::half + 1] * (tap<NC>(c + st) - tap<NC>(c - st));
-#pragma unroll
-      for (int j = 2; j <= S::half; ++j) s += cin[S::half + j] * (tap<NC>(c + j * st) - tap<NC>(c - j * st));
-      return s;
-    } else if (asym) {
-      double s = cin[0] * tap<NC>(c - S::half * st);
-#pragma unroll
-      for (int j = 1 - S::half; j <= S::half; ++j) s += cin[S::half + j] * tap<NC>(c + j * st);
-      return s;
-    } else {
-      double s = cin[S::half + 1] * (tap<NC>(c + st) + tap<NC>(c - st));
-#pragma unroll
-      for (int j = 2; j <= S::half; ++j) s += cin[S::half + j] * (tap<NC>(c + j * st) + tap<NC>(c - j * st));
-      return s + cin[S::half] * tap<NC>(c);
-    }
-  }
-  // periodic: interior stencil everywhere with wrapped indices
-  auto at = [&](int j) { return tap<NC>(line + (long long)wrapIndex(i + j, ax.n, ax.per) * st); };
-  if (asym) {
-    double s = cin[0] * at(-S::half);
-#pragma unroll
-    for (int j = 1 - S::half; j <= S::half; ++j) s += cin[S::half + j] * at(j);
+    for (int k = 1; k < S::width; ++k) s += __ldg(row + k) * tap<NC>(end + k * st);
     return s;
   }
-  if (S::skew) {
-    double s = cin[S::half + 1] * (at(1) - at(-1));
+  const double* __restrict__ row = &g_opLeft[ax.scheme][OP][m * S::width];
+  // right block = reflection of the left block, negated for skew operators
+  double s = __ldg(row + S::width - 1) * tap<NC>(end);
+#pragma unroll CU
+  for (int k = 1; k < S::width; ++k) s += __ldg(row + S::width - 1 - k) * tap<NC>(end + k * st);
+  return S::skew ? -s : s;
+}
+
+template <int OP>
+__device__ __forceinline__ bool inClosure(int i, const Axis& ax) {
+  return ax.per == 0 && (i < OpShape<OP>::depth || i >= ax.n - OpShape<OP>::depth);
+}
+
+// Taps p[j] = x_{i+j+1}, m[j] = x_{i-j-1} of the interior stencil; a periodic
+// line wraps near its ends only.
+template <int HALF, bool NC>
+__device__ __forceinline__ void interiorTaps(const double* __restrict__ c, int i, long long st, const Axis& ax,
+                                             double* p, double* m) {
+  if (i >= HALF && i < ax.n - HALF) {
 #pragma unroll
-    for (int j = 2; j <= S::half; ++j) s += cin[S::half + j] * (at(j) - at(-j));
-    return s;
+    for (int j = 1; j <= HALF; ++j) {
+      p[j - 1] = tap<NC>(c + j * st);
+      m[j - 1] = tap<NC>(c - j * st);
+    }
   } else {
-    double s = cin[S::half + 1] * (at(1) + at(-1));
+    const double* __restrict__ line = c - i * st;
 #pragma unroll
-    for (int j = 2; j <= S::half; ++j) s += cin[S::half + j] * (at(j) + at(-j));
-    return s + cin[S::half] * at(0);
+    for (int j = 1; j <= HALF; ++j) {
+      p[j - 1] = tap<NC>(line + (long long)wrapIndex(i + j, ax.n, ax.per) * st);
+      m[j - 1] = tap<NC>(line + (long long)wrapIndex(i - j, ax.n, ax.per) * st);
+    }
   }
+}
+
+// (Op x)_i along one axis; c points at the point itself, X: the axis of unit
+// stride.
+template <int OP, bool NC = true, int CU = 1, bool X = false>
+__device__ __forceinline__ double applyOp(const double* __restrict__ c, int i, const Axis& ax) {
+  using S = OpShape<OP>;
+  const long long st = X ? 1 : ax.stride;
+  if (inClosure<OP>(i, ax)) return closureSum<OP, NC, CU>(c, i, st, ax);
+  double p[S::half], m[S::half];
+  interiorTaps<S::half, NC>(c, i, st, ax, p, m);
+  if (!S::skew && (OP == OP_DISS || OP == OP_DISST) && c_ops.asym[ax.scheme][OP]) {
+    const double* __restrict__ cin = c_ops.interior[ax.scheme][OP];
+    double s = cin[0] * m[S::half - 1];
+#pragma unroll
+    for (int j = 1 - S::half; j <= S::half; ++j)
+      s += cin[S::half + j] * (j < 0 ? m[-j - 1] : (j > 0 ? p[j - 1] : tap<NC>(c)));
+    return s;
+  }
+  return interiorSum<OP>(p, m, S::skew ? 0.0 : tap<NC>(c), ax.scheme);
+}
+
+// Composite dissipation sum_d Dc_d x at a point, all axes' interior stencils
+// as one integer sum (they act on the same field, so one unit serves them):
+// one normalisation instead of one per axis. An axis whose closure holds the
+// point adds its FP64 row.
+template <int ND, bool NC, int CU>
+__device__ __forceinline__ double compositeDissipationSum(const double* __restrict__ c, const int* idx,
+                                                          const Axis* ax) {
+  double p[ND][4], m[ND][4], closure = 0.0;
+  const double x0 = tap<NC>(c);
+  int interior = 0;
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const long long st = d == 0 ? 1 : ax[d].stride;
+    if (inClosure<OP_DCOMP>(idx[d], ax[d])) {
+      closure += closureSum<OP_DCOMP, NC, CU>(c, idx[d], st, ax[d]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p[d][j] = m[d][j] = 0.0;
+    } else {
+      interiorTaps<4, NC>(c, idx[d], st, ax[d], p[d], m[d]);
+      ++interior;
+    }
+  }
+  if (interior == 0) return closure;
+  const int scheme = ax[0].scheme;
+  double s;
+  if (!(c_ops.fixed[scheme][OP_DCOMP].valid && fixedSymmetric<ND>(p, m, x0, interior, c_ops.fixed[scheme][OP_DCOMP], s))) {
+    const double* __restrict__ cin = c_ops.interior[scheme][OP_DCOMP];
+    s = (interior * cin[4]) * x0;
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s += cin[5 + j] * (p[d][j] + m[d][j]);
+  }
+  return interior == ND ? s : s + closure;
 }
 
 // x != 0.0 with integer operations: false for +0 and -0 only, as the

@@ -574,6 +574,7 @@ constexpr int kMaxExcitationModes = 256;  // modes of one solenoidal-excitation 
 // Blocks of the fixed-layout reductions (functional, sensitivity).
 int reductionBlocks(const DevBlock& b);
 void launchPowSelfTest(const double* x, int n, double e, double* fast, double* ref);
+void launchStencilSelfTest(const double* x, int n, int scheme, int op, double* out);
 Tile makeTile(const DevBlock& b, int tx, int ty, int tz);
 
 }  // namespace mgd

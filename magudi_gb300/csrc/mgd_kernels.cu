@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 
 #include "mgd_internal.h"
@@ -148,6 +149,30 @@ Tile makeTile(const DevBlock& b, int tx, int ty, int tz) {
 }
 
 
+// The integer form of an embedded operator's interior (mgd_fixed.cuh) over the
+// denominator den; valid = 0 when the coefficients do not have that form.
+static FixedOp fixedForm(const HostOp& h, int den) {
+  FixedOp f{};
+  const double s = h.I(1) < 0.0 ? -1.0 : 1.0;
+  f.flip = s < 0.0 ? 0x80000000u : 0u;
+  f.valid = 1;
+  for (int j = 0; j <= h.half; ++j) {
+    const double c = (j % 2 ? s : -s) * h.I(j) * den;
+    f.a[j] = (int)std::lround(c);
+    if (f.a[j] < 0 || f.a[j] > 1023 || std::fabs(c - f.a[j]) > 1e-12 || h.I(-j) != (h.skew && j ? -h.I(j) : h.I(j)))
+      f.valid = 0;
+  }
+  while ((1 << f.shift) < den) ++f.shift;
+  if (h.skew) {
+    --f.shift;  // 1/2 <= 2^shift / den < 1
+    f.rcp = (unsigned long long)std::llround(std::ldexp((long double)(1 << f.shift) / den, 63)) << 1;
+    if (f.a[0]) f.valid = 0;
+  } else if ((1 << f.shift) != den) {
+    f.valid = 0;
+  }
+  return f;
+}
+
 void uploadOperatorTables() {
   static bool done[64] = {false};
   int dev = 0;
@@ -178,6 +203,11 @@ void uploadOperatorTables() {
       for (size_t j = 0; j < h.right.size(); ++j) right[sc][o][j] = h.right[j];
       t.asym[sc][o] = h.asym ? 1 : 0;
     }
+    // common denominators of the schemes' interiors, in the order of MGD_SBP_*
+    static const int denD1[kSchemes] = {840, 2, 12, 60}, denComp[kSchemes] = {256, 2, 16, 64};
+    t.fixed[sc][OP_D1] = fixedForm(ops[OP_D1], denD1[sc]);
+    t.fixed[sc][OP_D1ADJ] = fixedForm(ops[OP_D1ADJ], denD1[sc]);
+    t.fixed[sc][OP_DCOMP] = fixedForm(ops[OP_DCOMP], denComp[sc]);
   }
   cudaMemcpyToSymbol(c_ops, &t, sizeof t);
   cudaMemcpyToSymbol(g_opLeft, left, sizeof left);
@@ -234,6 +264,29 @@ __device__ __forceinline__ bool locateAt(const BlockView& B, const Tile& T, int 
 
 __device__ __forceinline__ bool locate(const BlockView& B, const Tile& T, int b, long long& p, PointIndex& r) {
   return locateAt(B, T, b, threadIdx.x, p, r);
+}
+
+// f(std::integral_constant<int, d>) for every axis d: the axis of unit stride
+// is known at compile time.
+template <int ND, class F>
+__device__ __forceinline__ void forEachAxis(F f) {
+  f(std::integral_constant<int, 0>{});
+  if constexpr (ND > 1) f(std::integral_constant<int, 1>{});
+  if constexpr (ND > 2) f(std::integral_constant<int, 2>{});
+}
+
+// sum_d (Op_d x_d) at a point; x points at the point in the first axis' field,
+// the axes' fields lie `fieldStride` apart.
+template <int ND, int OP, bool NC = true>
+__device__ __forceinline__ double sumOverAxes(const double* x, long long fieldStride, const PointIndex& I,
+                                              const BlockView& B) {
+  double s = 0.0;
+  forEachAxis<ND>([&](auto axis) {
+    constexpr int d = decltype(axis)::value;
+    const double t = applyOp<OP, NC, kClosureUnroll<ND, NC>, d == 0>(x + fieldStride * d, I.idx[d], B.ax[d]);
+    s = d == 0 ? t : s + t;
+  });
+  return s;
 }
 
 // Primitive variables of one state (computeDependentVariables +
@@ -429,12 +482,11 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
     double du[ND][ND], dT[ND];
     if constexpr (LANES == 2) {
       const int d = lane;
-      const long long bd = d ? I.base[1] : I.base[0];
       const int id = d ? I.idx[1] : I.idx[0];
       const Axis ax = d ? B.ax[1] : B.ax[0];
-      const double a0 = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.u(0) + bd, id, ax);
-      const double a1 = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.u(1) + bd, id, ax);
-      const double aT = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.T() + bd, id, ax);
+      const double a0 = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.u(0) + p, id, ax);
+      const double a1 = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.u(1) + p, id, ax);
+      const double aT = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.T() + p, id, ax);
       const unsigned pair = 3u << (threadIdx.x & 30);
       const double b0 = __shfl_xor_sync(pair, a0, 1);
       const double b1 = __shfl_xor_sync(pair, a1, 1);
@@ -443,12 +495,13 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
       du[1][0] = d ? b1 : a1; du[1][1] = d ? a1 : b1;
       dT[0] = d ? bT : aT; dT[1] = d ? aT : bT;
     } else {
+      forEachAxis<ND>([&](auto axis) {
+        constexpr int d = decltype(axis)::value;
 #pragma unroll
-      for (int d = 0; d < ND; ++d) {
-#pragma unroll
-        for (int c = 0; c < ND; ++c) du[c][d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.u(c) + I.base[d], I.idx[d], B.ax[d]);
-        dT[d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.T() + I.base[d], I.idx[d], B.ax[d]);
-      }
+        for (int c = 0; c < ND; ++c)
+          du[c][d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.u(c) + p, I.idx[d], B.ax[d]);
+        dT[d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.T() + p, I.idx[d], B.ax[d]);
+      });
     }
     double gu[ND][ND], gT[ND];
     for (int x = 0; x < ND; ++x) {
@@ -614,13 +667,14 @@ __device__ __forceinline__ void dissipationPoint(const BlockView& B, const Physi
   const long long N = B.N;
   const double* x = src + N * c;
   if (P.composite) {
-    double s = applyOp<OP_DCOMP, NC, kClosureUnroll<ND, NC>>(x + I.base[0], I.idx[0], B.ax[0]);
-    for (int d = 1; d < ND; ++d) s += applyOp<OP_DCOMP, NC, kClosureUnroll<ND, NC>>(x + I.base[d], I.idx[d], B.ax[d]);
+    const double s = compositeDissipationSum<ND, NC, kClosureUnroll<ND, NC>>(x + p, I.idx, B.ax);
     B.dq[p + N * c] = (sign * P.dissipationAmount) * s;
   } else {
-    for (int d = 0; d < ND; ++d)
+    forEachAxis<ND>([&](auto axis) {
+      constexpr int d = decltype(axis)::value;
       B.dq[p + N * (d * nU + c)] =
-          (sign * B.arcA[p + N * d]) * applyOp<OP_DISS, NC, kClosureUnroll<ND, NC>>(x + I.base[d], I.idx[d], B.ax[d]);
+          (sign * B.arcA[p + N * d]) * applyOp<OP_DISS, NC, kClosureUnroll<ND, NC>, d == 0>(x + p, I.idx[d], B.ax[d]);
+    });
   }
 }
 
@@ -885,9 +939,7 @@ __device__ __forceinline__ double dissipationTerm(const BlockView& B, const Phys
   constexpr int nU = ND + 2;
   const long long N = B.N;
   if (P.composite) return B.dq[p + N * c];
-  double s = applyOp<OP_DISST, NC, kClosureUnroll<ND, NC>>(B.dq + N * c + I.base[0], I.idx[0], B.ax[0]);
-  for (int i = 1; i < ND; ++i) s += applyOp<OP_DISST, NC, kClosureUnroll<ND, NC>>(B.dq + N * (i * nU + c) + I.base[i], I.idx[i], B.ax[i]);
-  return s;
+  return sumOverAxes<ND, OP_DISST, NC>(B.dq + N * c + p, N * nU, I, B);
 }
 
 // ---------------------------------------------------------------------------
@@ -909,9 +961,7 @@ __device__ __forceinline__ void forwardDivergencePoint(const BlockView& B, const
   constexpr int nU = ND + 2, E = ND + 1;
   const int c = comp >= 0 ? comp : (int)blockIdx.y;
   const long long N = B.N;
-  double s = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.fhat + N * c + I.base[0], I.idx[0], B.ax[0]);
-  for (int i = 1; i < ND; ++i) s += applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.fhat + N * (i * nU + c) + I.base[i], I.idx[i], B.ax[i]);
-  double r = -s;
+  double r = -sumOverAxes<ND, OP_D1, NC>(B.fhat + N * c + p, N * nU, I, B);
   if (P.dissipation) r += dissipationTerm<ND, NC>(B, P, I, p, c);
   r = r * B.jac[p];
   for (int k = 0; k < 3; ++k) {
@@ -1192,7 +1242,8 @@ __global__ void __launch_bounds__(kBlock) kAdjointSatVectors(BlockView B, Physic
 // ad[j]. y and ad start from zero, so summing the directions' shares in
 // direction order reproduces the per-point accumulation exactly.
 template <int ND, bool CURV, bool VISC, int I>
-__device__ __forceinline__ void adjointCoreDirection(const BlockView& B, const Physics& P, const PointIndex& Ix,
+__device__ __forceinline__ void adjointCoreDirection(const BlockView& B, const Physics& P, long long p,
+                                                     const PointIndex& Ix,
                                                      const double* m, const double* u, double Tm, double v,
                                                      const double* tau, const double* hf, double mu, double la,
                                                      double kd, double jac, double* y, double (*ad)[ND + 1]) {
@@ -1200,7 +1251,8 @@ __device__ __forceinline__ void adjointCoreDirection(const BlockView& B, const P
   const long long N = B.N;
   double w[nU];
 #pragma unroll
-  for (int c = 0; c < nU; ++c) w[c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>>(B.lam + N * c + Ix.base[I], Ix.idx[I], B.ax[I]);
+  for (int c = 0; c < nU; ++c)
+    w[c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, I == 0>(B.lam + N * c + p, Ix.idx[I], B.ax[I]);
   for (int c = 0; c < nU; ++c) y[c] = 0.0;
   if (CURV) {
     addFluxJacobianTransposeProduct<ND, VISC>(m + ND * I, u, Tm, v, P, P.powerLawExponent, tau, hf, w, y);
@@ -1232,10 +1284,12 @@ __device__ __forceinline__ void adjointCorePoint(const BlockView& B, const Physi
   const PrimLayout L{ND};
   const FwdState fs = forwardState<ND>(B, rs, stage, fromSlot != 0);
   double w[ND][nU];
+  forEachAxis<ND>([&](auto axis) {
+    constexpr int i = decltype(axis)::value;
 #pragma unroll
-  for (int i = 0; i < ND; ++i)
-#pragma unroll
-    for (int c = 0; c < nU; ++c) w[i][c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>>(B.lam + N * c + I.base[i], I.idx[i], B.ax[i]);
+    for (int c = 0; c < nU; ++c)
+      w[i][c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, i == 0>(B.lam + N * c + p, I.idx[i], B.ax[i]);
+  });
   double m[ND * ND];
   for (int c = 0; c < ND * ND; ++c) m[c] = (CURV || (c % (ND + 1)) == 0) ? B.metrics[p + N * c] : 0.0;
   double u[ND];
@@ -1319,11 +1373,11 @@ __global__ void __launch_bounds__(2 * kMaxTile) kAdjointCoreSplit(BlockView B, P
     }
     double y[nU], ad[ND][nV];
     if (dir == 0)
-      adjointCoreDirection<ND, CURV, VISC, 0>(B, P, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
+      adjointCoreDirection<ND, CURV, VISC, 0>(B, P, p, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
     else if (ND > 1 && dir == 1)
-      adjointCoreDirection<ND, CURV, VISC, (ND > 1 ? 1 : 0)>(B, P, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
+      adjointCoreDirection<ND, CURV, VISC, (ND > 1 ? 1 : 0)>(B, P, p, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
     else
-      adjointCoreDirection<ND, CURV, VISC, (ND > 2 ? 2 : 0)>(B, P, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
+      adjointCoreDirection<ND, CURV, VISC, (ND > 2 ? 2 : 0)>(B, P, p, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
     double* mine = share + (long long)dir * K * TT + pt;
     for (int c = 0; c < nU; ++c) mine[c * TT] = y[c];
     if (VISC)
@@ -1366,9 +1420,7 @@ __device__ __forceinline__ void adjointDiffusionPoint(const BlockView& B, const 
   constexpr int nV = ND + 1;
   const int c = blockIdx.y;
   const long long N = B.N;
-  double s = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>>(B.ad + N * c + I.base[0], I.idx[0], B.ax[0]);
-  for (int j = 1; j < ND; ++j) s += applyOp<OP_D1ADJ, true, kClosureUnroll<ND>>(B.ad + N * (j * nV + c) + I.base[j], I.idx[j], B.ax[j]);
-  B.t2[p + N * c] = s;
+  B.t2[p + N * c] = sumOverAxes<ND, OP_D1ADJ>(B.ad + N * c + p, N * nV, I, B);
 }
 
 template <int ND>
@@ -1543,10 +1595,12 @@ __global__ void __launch_bounds__(kMaxTile) kLinearizedFlux(BlockView B, Physics
     la = fs.prim[p + N * L.la()];
     kd = fs.prim[p + N * L.k()];
     jac = B.jac[p];
+    forEachAxis<ND>([&](auto axis) {
+      constexpr int j = decltype(axis)::value;
 #pragma unroll
-    for (int j = 0; j < ND; ++j)
-#pragma unroll
-      for (int c = 0; c < nV; ++c) dt[j][c] = applyOp<OP_D1, true, kClosureUnroll<ND>>(B.t2 + N * c + I.base[j], I.idx[j], B.ax[j]);
+      for (int c = 0; c < nV; ++c)
+        dt[j][c] = applyOp<OP_D1, true, kClosureUnroll<ND>, j == 0>(B.t2 + N * c + p, I.idx[j], B.ax[j]);
+    });
   }
 #pragma unroll
   for (int i = 0; i < ND; ++i) {
@@ -2411,7 +2465,7 @@ __global__ void kCoordinateDerivative(BlockView B, const double* __restrict__ co
     const double* line = coords + B.N * c + I.base[dir];
     double s;
     if (ax.per != MGD_PERIODIC_PLANE) {
-      s = applyOp<OP_D1>(line, I.idx[dir], ax);
+      s = applyOp<OP_D1>(coords + B.N * c + p, I.idx[dir], ax);
     } else {
       const double* cin = c_ops.interior[ax.scheme][OP_D1];
       auto at = [&](int j) {
@@ -2435,7 +2489,7 @@ __global__ void kApplyD1(BlockView B, int dir, const double* __restrict__ in, do
   const long long p = (long long)blockIdx.x * kBlock + threadIdx.x;
   if (p >= B.N) return;
   const PointIndex I = pointIndex(B, p);
-  for (int c = 0; c < ncomp; ++c) out[p + B.N * c] = applyOp<OP_D1>(in + B.N * c + I.base[dir], I.idx[dir], B.ax[dir]);
+  for (int c = 0; c < ncomp; ++c) out[p + B.N * c] = applyOp<OP_D1>(in + B.N * c + p, I.idx[dir], B.ax[dir]);
 }
 
 // Far-field SAT matrices sigma_inv * (1/det) * A+(q_target, metric_normal).
@@ -2495,6 +2549,24 @@ __global__ void kPowSelfTest(const double* __restrict__ x, int n, double e, doub
   if (i >= n) return;
   fast[i] = fastPowPositive(x[i], e, &g_powTables);
   ref[i] = pow(x[i], e);
+}
+
+// Interior stencils of n windows of nine taps (offsets -4..4): op 0 the first
+// derivative, 1 its adjoint, 2 the composite dissipation.
+__global__ void kStencilSelfTest(const double* __restrict__ x, int n, int scheme, int op, double* __restrict__ out) {
+  const int i = blockIdx.x * kBlock + threadIdx.x;
+  if (i >= n) return;
+  const double* c = x + 9LL * i + 4;
+  const Axis ax{9, 1, 1, scheme};
+  const int idx = 4;
+  out[i] = op == 0   ? applyOp<OP_D1>(c, idx, ax)
+           : op == 1 ? applyOp<OP_D1ADJ>(c, idx, ax)
+                     : compositeDissipationSum<1, true, 1>(c, &idx, &ax);
+}
+
+void launchStencilSelfTest(const double* x, int n, int scheme, int op, double* out) {
+  uploadOperatorTables();
+  kStencilSelfTest<<<(n + kBlock - 1) / kBlock, kBlock>>>(x, n, scheme, op, out);
 }
 
 void launchPowSelfTest(const double* x, int n, double e, double* fast, double* ref) {
