@@ -1137,53 +1137,6 @@ __global__ void __launch_bounds__(kBlock) kGradientSensitivity(BlockView B, RunS
 // penalty (src/RhsHelperImpl.f90:89-250) folded into the same sweep, and
 // the complete far-field adjoint SAT vector (src/FarFieldPatchImpl.f90:237-257).
 // ---------------------------------------------------------------------------
-// The point's share of the adjoint core once the direction sums y (nU) and
-// ad (nD x (nU-1)) are formed: the far-field viscous adjoint penalty and the
-// interface terms added to ad, rcore and ad stored. The SAT vectors of the
-// wall and far-field entries come from kAdjointSatVectors.
-template <int ND, bool CURV, bool VISC>
-__device__ __forceinline__ void adjointCoreFinish(const BlockView& B, long long p, const FwdState& fs,
-                                                  const double* m, const double* u, const double* y,
-                                                  double (*ad)[ND + 1]) {
-  constexpr int nU = ND + 2, nV = ND + 1;
-  const long long N = B.N;
-  const PrimLayout L{ND};
-  for (int c = 0; c < nU; ++c) B.rcore[p + N * c] = y[c];
-  double lp[nU];
-  for (int c = 0; c < nU; ++c) lp[c] = B.lam[p + N * c];
-  const double jac = B.jac[p];
-  if (VISC) {
-    const double mu = fs.prim[p + N * L.mu()], la = fs.prim[p + N * L.la()], kd = fs.prim[p + N * L.k()];
-    for (int k = 0; k < 3; ++k) {
-      const int e = B.ffOfPoint[3 * p + k];
-      if (e < 0 || B.ff.kind[e] != SAT_FAR_FIELD) continue;
-      const int nd = B.ff.normalDir[e] - 1;
-      double mn[ND];  // metric row of the normal direction, read from memory (no dynamic register index)
-      for (int d = 0; d < ND; ++d) mn[d] = CURV || d == nd ? B.metrics[p + N * (ND * nd + d)] : 0.0;
-      const double sv = B.ff.sigVRaw[e];
-      for (int l = 0; l < ND; ++l) {
-        double t[nV];
-        for (int c = 0; c < nV; ++c) t[c] = 0.0;
-        if (CURV)
-          secondPartialViscousTransposeProduct<ND>(u, mu, la, kd, jac, mn, m + ND * l, &lp[1], t);
-        else
-          secondPartialViscousTransposeProductCart<ND>(u, mu, la, kd, jac, nd, B.metrics[p + N * (ND * nd + nd)], l,
-                                                       m[ND * l + l], &lp[1], t);
-        for (int c = 0; c < nV; ++c) ad[l][c] += sv * t[c];
-      }
-    }
-    for (int k = 0; k < 3; ++k) {
-      const int e = B.ffOfPoint[3 * p + k];
-      if (e < 0 || B.ff.kind[e] != SAT_INTERFACE) continue;
-      const double* a = B.ff.ifAd + (long long)e * ND * nV;
-      for (int l = 0; l < ND; ++l)
-        for (int c = 0; c < nV; ++c) ad[l][c] += a[l * nV + c];
-    }
-    for (int j = 0; j < ND; ++j)
-      for (int c = 0; c < nV; ++c) B.ad[p + N * (j * nV + c)] = ad[j][c];
-  }
-}
-
 // The adjoint SAT vector of every wall and far-field entry (B.ff.visc), one
 // thread per entry: the far-field adjoint SAT (src/FarFieldPatchImpl.f90:
 // 237-257) and the wall SATs (src/ImpenetrableWallImpl.f90,
@@ -1237,39 +1190,77 @@ __global__ void __launch_bounds__(kBlock) kAdjointSatVectors(BlockView B, Physic
   }
 }
 
-// One direction's share of the adjoint core at a point: w = D+_I lambda, the
-// (A_I - B1_I)^T w product into y and the B2(m_I, m_j)^T w products into
-// ad[j]. y and ad start from zero, so summing the directions' shares in
-// direction order reproduces the per-point accumulation exactly.
-template <int ND, bool CURV, bool VISC, int I>
-__device__ __forceinline__ void adjointCoreDirection(const BlockView& B, const Physics& P, long long p,
-                                                     const PointIndex& Ix,
-                                                     const double* m, const double* u, double Tm, double v,
-                                                     const double* tau, const double* hf, double mu, double la,
-                                                     double kd, double jac, double* y, double (*ad)[ND + 1]) {
+// D+_I lambda of every component at a point.
+template <int ND, int I>
+__device__ __forceinline__ void adjointDerivative(const BlockView& B, long long p, const PointIndex& Ix, double* w) {
+  const long long N = B.N;
+#pragma unroll
+  for (int c = 0; c < ND + 2; ++c)
+    w[c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, I == 0>(B.lam + N * c + p, Ix.idx[I], B.ax[I]);
+}
+
+// The point's core from the adjoint derivatives w along every axis: rcore
+// and the viscous diffusion ad stored, the far-field viscous penalty and the
+// interface terms included. The SAT vectors of the wall and far-field entries
+// come from kAdjointSatVectors.
+template <int ND, bool CURV, bool VISC>
+__device__ __forceinline__ void adjointCoreFrom(const BlockView& B, const Physics& P, const FwdState& fs, long long p,
+                                                const double (*w)[ND + 2]) {
   constexpr int nU = ND + 2, nV = ND + 1;
   const long long N = B.N;
-  double w[nU];
-#pragma unroll
-  for (int c = 0; c < nU; ++c)
-    w[c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, I == 0>(B.lam + N * c + p, Ix.idx[I], B.ax[I]);
-  for (int c = 0; c < nU; ++c) y[c] = 0.0;
-  if (CURV) {
-    addFluxJacobianTransposeProduct<ND, VISC>(m + ND * I, u, Tm, v, P, P.powerLawExponent, tau, hf, w, y);
-  } else {
-    const double nTv = VISC ? P.powerLawExponent * P.g * v / Tm : 0.0;
-    addFluxJacobianTransposeProductCart<ND, VISC>(I, m[ND * I + I], u, Tm, v, P, nTv, tau, hf, w, y);
-  }
+  const PrimLayout L{ND};
+  double m[ND * ND];
+  for (int c = 0; c < ND * ND; ++c) m[c] = (CURV || (c % (ND + 1)) == 0) ? B.metrics[p + N * c] : 0.0;
+  double u[ND];
+  for (int d = 0; d < ND; ++d) u[d] = fs.prim[p + N * L.u(d)];
+  const double v = fs.prim[p + N * L.v()], Tm = fs.prim[p + N * L.T()];
+  double tau[ND * ND], hf[ND], mu = 0.0, la = 0.0, kd = 0.0, jac = 0.0;
   if (VISC) {
+    for (int c = 0; c < ND * ND; ++c) tau[c] = fs.tau[p + N * c];
+    for (int d = 0; d < ND; ++d) hf[d] = fs.hf[p + N * d];
+    mu = fs.prim[p + N * L.mu()];
+    la = fs.prim[p + N * L.la()];
+    kd = fs.prim[p + N * L.k()];
+    jac = B.jac[p];
+  }
+  // the far-field viscous adjoint penalty sum_l D+_l (sigma B2(m_n, m_l)^T lambda)
+  // (src/RhsHelperImpl.f90:89-250) joins the diffusion as if sigma lambda were
+  // part of the adjoint derivative along the entry's normal n
+  auto farFieldPenalty = [&](double (*W)[nU]) -> bool {
+    bool any = false;
+    for (int k = 0; k < 3; ++k) {
+      const int e = B.ffOfPoint[3 * p + k];
+      if (e < 0 || B.ff.kind[e] != SAT_FAR_FIELD) continue;
+      any = true;
+      const int nd = B.ff.normalDir[e] - 1;
+      const double sv = B.ff.sigVRaw[e];
+      double lp[nU];
 #pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      for (int c = 0; c < nV; ++c) ad[j][c] = 0.0;
-      if (CURV)
-        secondPartialViscousTransposeProduct<ND>(u, mu, la, kd, jac, m + ND * I, m + ND * j, &w[1], ad[j]);
-      else
-        secondPartialViscousTransposeProductCart<ND>(u, mu, la, kd, jac, I, m[ND * I + I], j, m[ND * j + j], &w[1],
-                                                     ad[j]);
+      for (int c = 1; c < nU; ++c) lp[c] = B.lam[p + N * c];
+#pragma unroll
+      for (int x = 0; x < ND; ++x) {
+        // the metric row of the normal direction, read from memory (no dynamic register index)
+        if (!CURV && x != nd) continue;
+        const double f = sv * B.metrics[p + N * (ND * nd + x)];
+#pragma unroll
+        for (int c = 1; c < nU; ++c) W[x][c] += f * lp[c];
+      }
     }
+    return any;
+  };
+  double y[nU], ad[ND][nV];
+  adjointPointwise<ND, CURV, VISC>(w, m, u, Tm, v, P, tau, hf, mu, la, kd, jac, farFieldPenalty, y, ad);
+  for (int c = 0; c < nU; ++c) B.rcore[p + N * c] = y[c];
+  if (VISC) {
+    for (int k = 0; k < 3; ++k) {
+      const int e = B.ffOfPoint[3 * p + k];
+      if (e < 0 || B.ff.kind[e] != SAT_INTERFACE) continue;
+      const double* a = B.ff.ifAd + (long long)e * ND * nV;
+      for (int l = 0; l < ND; ++l)
+        for (int c = 0; c < nV; ++c) ad[l][c] += a[l * nV + c];
+    }
+    for (int j = 0; j < ND; ++j)
+      for (int c = 0; c < nV; ++c) B.ad[p + N * (j * nV + c)] = ad[j][c];
   }
 }
 
@@ -1279,128 +1270,45 @@ __device__ __forceinline__ void adjointCorePoint(const BlockView& B, const Physi
   long long p;
   PointIndex I;
   if (!locate(B, T, blk, p, I)) return;
-  constexpr int nU = ND + 2, nV = ND + 1;
-  const long long N = B.N;
-  const PrimLayout L{ND};
   const FwdState fs = forwardState<ND>(B, rs, stage, fromSlot != 0);
-  double w[ND][nU];
+  double w[ND][ND + 2];
   forEachAxis<ND>([&](auto axis) {
     constexpr int i = decltype(axis)::value;
-#pragma unroll
-    for (int c = 0; c < nU; ++c)
-      w[i][c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, i == 0>(B.lam + N * c + p, I.idx[i], B.ax[i]);
+    adjointDerivative<ND, i>(B, p, I, w[i]);
   });
-  double m[ND * ND];
-  for (int c = 0; c < ND * ND; ++c) m[c] = (CURV || (c % (ND + 1)) == 0) ? B.metrics[p + N * c] : 0.0;
-  double u[ND];
-  for (int d = 0; d < ND; ++d) u[d] = fs.prim[p + N * L.u(d)];
-  const double v = fs.prim[p + N * L.v()], Tm = fs.prim[p + N * L.T()];
-  double tau[ND * ND], hf[ND];
-  if (VISC) {
-    for (int c = 0; c < ND * ND; ++c) tau[c] = fs.tau[p + N * c];
-    for (int d = 0; d < ND; ++d) hf[d] = fs.hf[p + N * d];
-  }
-  double y[nU];
-  for (int c = 0; c < nU; ++c) y[c] = 0.0;
-  if (CURV) {
-#pragma unroll
-    for (int i = 0; i < ND; ++i)
-      addFluxJacobianTransposeProduct<ND, VISC>(m + ND * i, u, Tm, v, P, P.powerLawExponent, tau, hf, w[i], y);
-  } else {
-    const double nTv = VISC ? P.powerLawExponent * P.g * v / Tm : 0.0;
-#pragma unroll
-    for (int i = 0; i < ND; ++i)
-      addFluxJacobianTransposeProductCart<ND, VISC>(i, m[ND * i + i], u, Tm, v, P, nTv, tau, hf, w[i], y);
-  }
-  double ad[ND][nV];
-  if (VISC) {
-    const double mu = fs.prim[p + N * L.mu()], la = fs.prim[p + N * L.la()], kd = fs.prim[p + N * L.k()];
-    const double jac = B.jac[p];
-#pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      for (int c = 0; c < nV; ++c) ad[j][c] = 0.0;
-#pragma unroll
-      for (int i = 0; i < ND; ++i) {
-        if (CURV)
-          secondPartialViscousTransposeProduct<ND>(u, mu, la, kd, jac, m + ND * i, m + ND * j, &w[i][1], ad[j]);
-        else
-          secondPartialViscousTransposeProductCart<ND>(u, mu, la, kd, jac, i, m[ND * i + i], j, m[ND * j + j],
-                                                       &w[i][1], ad[j]);
-      }
-    }
-  }
-  adjointCoreFinish<ND, CURV, VISC>(B, p, fs, m, u, y, ad);
+  adjointCoreFrom<ND, CURV, VISC>(B, P, fs, p, w);
 }
 
-// The adjoint core with nD threads per point: thread block = tile threads x
-// nD, thread (point, direction I) forms its direction's share
-// (adjointCoreDirection), the shares meet in shared memory and the
-// direction-0 thread of each point sums them in direction order and finishes
-// the point. Twice (2D) the threads of the per-point kernel, each with a
-// third of its stencil work, for grids too small to fill the GPU per point.
+// The adjoint core with nD threads per point (2D): thread block = tile
+// threads x nD, thread (point, direction i) forms the adjoint derivatives
+// along its axis, they meet in shared memory and the direction-0 thread of
+// each point forms the point's core. Twice the threads of the per-point
+// kernel for the stencils, for grids too small to fill the GPU per point.
 template <int ND, bool CURV, bool VISC>
 __global__ void __launch_bounds__(2 * kMaxTile) kAdjointCoreSplit(BlockView B, Physics P, RunScalars rs, int stage,
                                                                  int fromSlot, Tile T) {
+  static_assert(ND == 2, "two directions");
   pdlEnter();
-  constexpr int nU = ND + 2, nV = ND + 1, K = nU + ND * nV;
-  extern __shared__ double share[];
+  constexpr int nU = ND + 2;
+  extern __shared__ double share[];  // direction 1's derivatives: nU x tile threads
   const int TT = T.threads();
   const int pt = threadIdx.x % TT, dir = threadIdx.x / TT;
   long long p = 0;
   PointIndex I;
   const bool ok = locateAt(B, T, blockIdx.x, pt, p, I);
-  const long long N = B.N;
-  const PrimLayout L{ND};
-  FwdState fs{};
-  double m[ND * ND], u[ND], tau[ND * ND], hf[ND];
-  double v = 0.0, Tm = 0.0;
+  double w[ND][nU];
   if (ok) {
-    fs = forwardState<ND>(B, rs, stage, fromSlot != 0);
-    for (int c = 0; c < ND * ND; ++c) m[c] = (CURV || (c % (ND + 1)) == 0) ? B.metrics[p + N * c] : 0.0;
-    for (int d = 0; d < ND; ++d) u[d] = fs.prim[p + N * L.u(d)];
-    v = fs.prim[p + N * L.v()];
-    Tm = fs.prim[p + N * L.T()];
-    if (VISC) {
-      for (int c = 0; c < ND * ND; ++c) tau[c] = fs.tau[p + N * c];
-      for (int d = 0; d < ND; ++d) hf[d] = fs.hf[p + N * d];
+    if (dir == 0) {
+      adjointDerivative<ND, 0>(B, p, I, w[0]);
+    } else {
+      adjointDerivative<ND, 1>(B, p, I, w[1]);
+      for (int c = 0; c < nU; ++c) share[c * TT + pt] = w[1][c];
     }
-    double mu = 0.0, la = 0.0, kd = 0.0, jac = 0.0;
-    if (VISC) {
-      mu = fs.prim[p + N * L.mu()];
-      la = fs.prim[p + N * L.la()];
-      kd = fs.prim[p + N * L.k()];
-      jac = B.jac[p];
-    }
-    double y[nU], ad[ND][nV];
-    if (dir == 0)
-      adjointCoreDirection<ND, CURV, VISC, 0>(B, P, p, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
-    else if (ND > 1 && dir == 1)
-      adjointCoreDirection<ND, CURV, VISC, (ND > 1 ? 1 : 0)>(B, P, p, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
-    else
-      adjointCoreDirection<ND, CURV, VISC, (ND > 2 ? 2 : 0)>(B, P, p, I, m, u, Tm, v, tau, hf, mu, la, kd, jac, y, ad);
-    double* mine = share + (long long)dir * K * TT + pt;
-    for (int c = 0; c < nU; ++c) mine[c * TT] = y[c];
-    if (VISC)
-      for (int j = 0; j < ND; ++j)
-        for (int c = 0; c < nV; ++c) mine[(nU + j * nV + c) * TT] = ad[j][c];
   }
   __syncthreads();
   if (!ok || dir != 0) return;
-  double y[nU], ad[ND][nV];
-  for (int c = 0; c < nU; ++c) {
-    double t = share[c * TT + pt];
-    for (int i = 1; i < ND; ++i) t += share[((long long)i * K + c) * TT + pt];
-    y[c] = t;
-  }
-  if (VISC)
-    for (int j = 0; j < ND; ++j)
-      for (int c = 0; c < nV; ++c) {
-        const int k = nU + j * nV + c;
-        double t = share[k * TT + pt];
-        for (int i = 1; i < ND; ++i) t += share[((long long)i * K + k) * TT + pt];
-        ad[j][c] = t;
-      }
-  adjointCoreFinish<ND, CURV, VISC>(B, p, fs, m, u, y, ad);
+  for (int c = 0; c < nU; ++c) w[1][c] = share[c * TT + pt];
+  adjointCoreFrom<ND, CURV, VISC>(B, P, forwardState<ND>(B, rs, stage, fromSlot != 0), p, w);
 }
 
 template <int ND, bool CURV, bool VISC>
@@ -2730,8 +2638,8 @@ void launchAdjointCore(Context& c, DevBlock& b, const RunScalars& rs, int stage,
   const bool curv = b.v.curvilinear != 0, visc = c.phys.viscous != 0;
   MGD_LAUNCH(c);
   if (b.coreLanes == 2 && c.nD == 2) {
-    // nD threads per point; their shares meet in shared memory
-    const size_t smem = (size_t)2 * (4 + 2 * 3) * W * sizeof(double);
+    // nD threads per point; the second direction's derivatives pass through shared memory
+    const size_t smem = (size_t)4 * W * sizeof(double);
 #define ACS(CU, VI) pdlShared(kAdjointCoreSplit<2, CU, VI>, G, 2 * W, smem, st, b.v, c.phys, rs, stage, fromSlot, T)
     if (curv) { if (visc) ACS(true, true); else ACS(true, false); }
     else { if (visc) ACS(false, true); else ACS(false, false); }
