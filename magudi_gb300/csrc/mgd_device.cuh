@@ -325,14 +325,20 @@ template <int K> __host__ __device__ inline DualN<K> operator*(const DualN<K>& a
   return r;
 }
 template <int K> __host__ __device__ inline DualN<K> operator/(const DualN<K>& a, const DualN<K>& b) {
-  DualN<K> r(a.v / b.v);
-  for (int k = 0; k < K; ++k) r.d[k] = (a.d[k] * b.v - a.v * b.d[k]) / (b.v * b.v);
+  // one FP64 division (about ten instructions) for the value and the derivatives
+  const double inv = 1.0 / b.v;
+  DualN<K> r(a.v * inv);
+  for (int k = 0; k < K; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * inv;
   return r;
 }
-template <int K> __host__ __device__ inline DualN<K> operator+(const DualN<K>& a, double b) { return a + DualN<K>(b); }
-template <int K> __host__ __device__ inline DualN<K> operator+(double a, const DualN<K>& b) { return DualN<K>(a) + b; }
-template <int K> __host__ __device__ inline DualN<K> operator-(const DualN<K>& a, double b) { return a - DualN<K>(b); }
-template <int K> __host__ __device__ inline DualN<K> operator-(double a, const DualN<K>& b) { return DualN<K>(a) - b; }
+template <int K> __host__ __device__ inline DualN<K> operator+(const DualN<K>& a, double b) {
+  DualN<K> r(a);
+  r.v += b;
+  return r;
+}
+template <int K> __host__ __device__ inline DualN<K> operator+(double a, const DualN<K>& b) { return b + a; }
+template <int K> __host__ __device__ inline DualN<K> operator-(const DualN<K>& a, double b) { return a + (-b); }
+template <int K> __host__ __device__ inline DualN<K> operator-(double a, const DualN<K>& b) { return (-b) + a; }
 template <int K> __host__ __device__ inline DualN<K> operator*(const DualN<K>& a, double b) {
   DualN<K> r(a.v * b);
   for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * b;
@@ -340,7 +346,12 @@ template <int K> __host__ __device__ inline DualN<K> operator*(const DualN<K>& a
 }
 template <int K> __host__ __device__ inline DualN<K> operator*(double a, const DualN<K>& b) { return b * a; }
 template <int K> __host__ __device__ inline DualN<K> operator/(const DualN<K>& a, double b) { return a / DualN<K>(b); }
-template <int K> __host__ __device__ inline DualN<K> operator/(double a, const DualN<K>& b) { return DualN<K>(a) / b; }
+template <int K> __host__ __device__ inline DualN<K> operator/(double a, const DualN<K>& b) {
+  const double inv = 1.0 / b.v;
+  DualN<K> r(a * inv);
+  for (int k = 0; k < K; ++k) r.d[k] = -(r.v * b.d[k]) * inv;
+  return r;
+}
 template <int K> __host__ __device__ inline DualN<K>& operator+=(DualN<K>& a, const DualN<K>& b) {
   a = a + b;
   return a;
@@ -348,29 +359,132 @@ template <int K> __host__ __device__ inline DualN<K>& operator+=(DualN<K>& a, co
 __host__ __device__ inline double sqrtOf(double x) { return sqrt(x); }
 template <int K> __host__ __device__ inline DualN<K> sqrtOf(const DualN<K>& a) {
   DualN<K> r(::sqrt(a.v));
-  for (int k = 0; k < K; ++k) r.d[k] = a.d[k] / (2.0 * r.v);
+  const double h = 0.5 / r.v;
+  for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * h;
   return r;
 }
 
 // Roe average of two conserved states (computeRoeAverage,
-// src/CNSHelperImpl.f90:179-351, without the variations).
-template <int ND, class S>
-__host__ __device__ inline void roeAverage(const S* qL, const S* qR, double g, S* roe) {
-  const S sL = sqrtOf(qL[0]), sR = sqrtOf(qR[0]);
-  const S vL = 1.0 / qL[0], vR = 1.0 / qR[0];
-  S mL2 = qL[1] * qL[1], mR2 = qR[1] * qR[1];
+// src/CNSHelperImpl.f90:179-351, without the variations). Of dual numbers, the
+// right state may be plain (not differentiated).
+template <int ND, class S, class SR>
+__host__ __device__ inline void roeAverage(const S* qL, const SR* qR, double g, S* roe) {
+  const S sL = sqrtOf(qL[0]);
+  const SR sR = sqrtOf(qR[0]);
+  const S vL = 1.0 / qL[0], w = 1.0 / (sL + sR);
+  const SR vR = 1.0 / qR[0];
+  S mL2 = qL[1] * qL[1];
+  SR mR2 = qR[1] * qR[1];
   for (int d = 1; d < ND; ++d) {
     mL2 = mL2 + qL[1 + d] * qL[1 + d];
     mR2 = mR2 + qR[1 + d] * qR[1 + d];
   }
   const S hL = g * qL[ND + 1] - 0.5 * (g - 1.0) * vL * mL2;
-  const S hR = g * qR[ND + 1] - 0.5 * (g - 1.0) * vR * mR2;
+  const SR hR = g * qR[ND + 1] - 0.5 * (g - 1.0) * vR * mR2;
   roe[0] = sL * sR;
-  for (int d = 0; d < ND; ++d) roe[1 + d] = (sR * qL[1 + d] + sL * qR[1 + d]) / (sL + sR);
-  roe[ND + 1] = (sR * hL + sL * hR) / (sL + sR);
+  for (int d = 0; d < ND; ++d) roe[1 + d] = (sR * qL[1 + d] + sL * qR[1 + d]) * w;
+  roe[ND + 1] = (sR * hL + sL * hR) * w;
   S m2 = roe[1] * roe[1];
   for (int d = 1; d < ND; ++d) m2 = m2 + roe[1 + d] * roe[1 + d];
-  roe[ND + 1] = (roe[ND + 1] + 0.5 * (g - 1.0) / roe[0] * m2) / g;
+  roe[ND + 1] = (roe[ND + 1] + 0.5 * (g - 1.0) / roe[0] * m2) * (1.0 / g);
+}
+
+// The incoming Jacobian A+ of incomingJacobian below without its matrix. With
+// n the unit normal, k = |u|^2/2, eigenvalues a (entropy and shear) and b+, b-
+// (acoustic; those of the other direction are zero), and for a vector x
+//   y = x_m - u x_0,  X = (k x_0 - u . x_m + x_E) / T,  w+- = (X +- n.y / c) / 2,
+// its eigenvector expansion sums to
+//   A+ x = a (x_0 - X, u (x_0 - X) + y - n (n.y), k (x_0 - X) + u.y - U (n.y))
+//          + sum+- b+- w+- (1, u +- n c, T + k +- c U).
+template <int ND, class S>
+struct Incoming {
+  S u[ND], T, iT, k, U, c, ic, a, bp, bm;
+  double n[ND];
+};
+
+template <int ND, class S>
+__host__ __device__ inline Incoming<ND, S> incomingState(const S* cv, const double* metrics, double g, int direction) {
+  Incoming<ND, S> I;
+  double arc = 0.0;
+  for (int d = 0; d < ND; ++d) arc += metrics[d] * metrics[d];
+  arc = sqrt(arc);
+  const double arcInv = 1.0 / arc;
+  for (int d = 0; d < ND; ++d) I.n[d] = metrics[d] * arcInv;
+  const S v = 1.0 / cv[0];
+  for (int d = 0; d < ND; ++d) I.u[d] = v * cv[1 + d];
+  S u2 = I.u[0] * I.u[0];
+  I.U = I.n[0] * I.u[0];
+  for (int d = 1; d < ND; ++d) {
+    u2 = u2 + I.u[d] * I.u[d];
+    I.U = I.U + I.n[d] * I.u[d];
+  }
+  I.k = 0.5 * u2;
+  I.T = g * (v * cv[ND + 1] - I.k);
+  I.c = sqrtOf((g - 1.0) * I.T);
+  I.ic = 1.0 / I.c;
+  I.iT = (g - 1.0) * I.ic * I.ic;
+  I.a = arc * I.U;
+  I.bp = arc * (I.U + I.c);
+  I.bm = arc * (I.U - I.c);
+  if (direction * valueOf(I.a) < 0.0) I.a = S(0.0);
+  if (direction * valueOf(I.bp) < 0.0) I.bp = S(0.0);
+  if (direction * valueOf(I.bm) < 0.0) I.bm = S(0.0);
+  return I;
+}
+
+// out = A+ x.
+template <int ND, class S>
+__host__ __device__ inline void incomingProduct(const Incoming<ND, S>& I, const double* x, S* out) {
+  constexpr int E = ND + 1;
+  S um = I.u[0] * x[1];
+  for (int d = 1; d < ND; ++d) um = um + I.u[d] * x[1 + d];
+  const S X = I.iT * (I.k * x[0] - um + x[E]);
+  S y[ND], ny = S(0.0), uy = S(0.0);
+  for (int d = 0; d < ND; ++d) {
+    y[d] = x[1 + d] - I.u[d] * x[0];
+    ny = d ? ny + I.n[d] * y[d] : I.n[0] * y[0];
+    uy = d ? uy + I.u[d] * y[d] : I.u[0] * y[0];
+  }
+  const S s = x[0] - X, wp = 0.5 * I.bp * (X + I.ic * ny), wm = 0.5 * I.bm * (X - I.ic * ny);
+  const S sum = wp + wm, dif = I.c * (wp - wm), as = I.a * s;
+  out[0] = as + sum;
+  for (int d = 0; d < ND; ++d) out[1 + d] = I.u[d] * out[0] + I.a * (y[d] - I.n[d] * ny) + I.n[d] * dif;
+  out[E] = I.k * out[0] + I.a * (uy - I.U * ny) + I.T * sum + I.U * dif;
+}
+
+// lam^T A+ x, and with grad != nullptr its gradient A+^T lam with respect to
+// x (values only):
+//   a [C (x_0 - X) + q.y - (n.q)(n.y)] + sum+- b+- (A +- c n.q) w+-,
+//   q = lam_m + u lam_E, C = lam_0 + u . lam_m + k lam_E, A = C + T lam_E.
+template <int ND, class S>
+__host__ __device__ inline S incomingForm(const Incoming<ND, S>& I, const double* lam, const double* x, double* grad) {
+  constexpr int E = ND + 1;
+  S q[ND], y[ND], nq = S(0.0), ny = S(0.0), qy = S(0.0), um = S(0.0), C = I.k * lam[E] + lam[0];
+  for (int d = 0; d < ND; ++d) {
+    q[d] = I.u[d] * lam[E] + lam[1 + d];
+    y[d] = x[1 + d] - I.u[d] * x[0];
+    C = C + I.u[d] * lam[1 + d];
+    um = d ? um + I.u[d] * x[1 + d] : I.u[0] * x[1];
+    nq = d ? nq + I.n[d] * q[d] : I.n[0] * q[0];
+    ny = d ? ny + I.n[d] * y[d] : I.n[0] * y[0];
+    qy = d ? qy + q[d] * y[d] : q[0] * y[0];
+  }
+  const S X = I.iT * (I.k * x[0] - um + x[E]), A = C + I.T * lam[E], cq = I.c * nq, cy = I.ic * ny;
+  const S hp = 0.5 * I.bp * (A + cq), hm = 0.5 * I.bm * (A - cq);
+  if (grad) {
+    const double gX = valueOf(hp) + valueOf(hm) - valueOf(I.a) * valueOf(C);
+    const double gn = (valueOf(hp) - valueOf(hm)) * valueOf(I.ic) - valueOf(I.a) * valueOf(nq);
+    const double gi = valueOf(I.iT) * gX;
+    double ug = 0.0;
+    for (int d = 0; d < ND; ++d) {
+      const double gy = valueOf(I.a) * valueOf(q[d]) + I.n[d] * gn;
+      grad[1 + d] = gy - gi * valueOf(I.u[d]);
+      ug += valueOf(I.u[d]) * gy;
+    }
+    grad[0] = valueOf(I.a) * valueOf(C) + gi * valueOf(I.k) - ug;
+    grad[E] = gi;
+  }
+  return I.a * (C * (x[0] - X) + qy - nq * ny) + hp * (X + cy) + hm * (X - cy);
 }
 
 template <int ND, class S = double>

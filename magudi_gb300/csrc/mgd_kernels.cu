@@ -1784,15 +1784,15 @@ __global__ void __launch_bounds__(kBlock) kInterfaceSat(BlockView B, Physics P, 
   const long long N = B.N, p = B.ff.point[e];
   const int pb = B.ff.partnerBlock[e];
   const long long pp = B.ff.partnerPoint[e], NR = R.N[pb];
-  double qL[nU], qR[nU], dq[nU], mL[ND], roe[nU], A[nU * nU];
+  double qL[nU], qR[nU], dq[nU], mL[ND], roe[nU], Ax[nU];
   for (int c = 0; c < nU; ++c) {
     qL[c] = B.q[p + N * c];
     qR[c] = R.q[pb][pp + NR * c];
     dq[c] = qL[c] - qR[c];
   }
   for (int d = 0; d < ND; ++d) mL[d] = B.metrics[p + N * (ND * (B.ff.normalDir[e] - 1) + d)];
-  roeAverage<ND, double>(qL, qR, P.g, roe);
-  incomingJacobian<ND, double>(roe, mL, P.g, B.ff.dirL[e], A);
+  roeAverage<ND, double, double>(qL, qR, P.g, roe);
+  incomingProduct<ND, double>(incomingState<ND, double>(roe, mL, P.g, B.ff.dirL[e]), dq, Ax);
   const double jac = B.jac[p];
   const double s = B.ff.ifInv[2 * e];
   double* sat = B.ff.visc + (long long)e * nU;
@@ -1805,9 +1805,7 @@ __global__ void __launch_bounds__(kBlock) kInterfaceSat(BlockView B, Physics P, 
   const double* fL = B.ff.ifVisc + (long long)e * nU;
   const double* fR = R.ifVisc[pb] + (long long)B.ff.partnerEntry[e] * nU;
   for (int r = 0; r < nU; ++r) {
-    double t = A[r] * dq[0];
-    for (int c = 1; c < nU; ++c) t += A[r + nU * c] * dq[c];
-    double v = -(s * jac * t);
+    double v = -(s * jac * Ax[r]);
     if (VISC && r > 0) v += jac * (vL * fL[r] + vR * fR[r]);
     sat[r] = v;
   }
@@ -1849,9 +1847,13 @@ __global__ void __launch_bounds__(kBlock) kInterfaceSatLinearized(BlockView B, P
     dR[c].d[0] = xR;
   }
   for (int d = 0; d < ND; ++d) mL[d] = B.metrics[p + N * (ND * (B.ff.normalDir[e] - 1) + d)];
-  roeAverage<ND, D>(dL, dR, P.g, roe);
-  D A[nU * nU];
-  incomingJacobian<ND, D>(roe, mL, P.g, B.ff.dirL[e], A);
+  roeAverage<ND, D, D>(dL, dR, P.g, roe);
+  // A+ dx on the values, the derivative of A+ dq on the duals
+  D Adq[nU];
+  double vroe[nU], Adx[nU];
+  for (int c = 0; c < nU; ++c) vroe[c] = roe[c].v;
+  incomingProduct<ND, D>(incomingState<ND, D>(roe, mL, P.g, B.ff.dirL[e]), dq, Adq);
+  incomingProduct<ND, double>(incomingState<ND, double>(vroe, mL, P.g, B.ff.dirL[e]), dx, Adx);
   const double jac = B.jac[p];
   const double s = B.ff.ifInv[2 * e];
   double vL = 0.0, vR = 0.0;
@@ -1864,12 +1866,7 @@ __global__ void __launch_bounds__(kBlock) kInterfaceSatLinearized(BlockView B, P
   const double* fR = R.ifVisc[pb] + (long long)B.ff.partnerEntry[e] * nU;
   double* sat = B.ff.visc + (long long)e * nU;
   for (int r = 0; r < nU; ++r) {
-    double t1 = A[r].v * dx[0], t2 = A[r].d[0] * dq[0];
-    for (int c = 1; c < nU; ++c) {
-      t1 += A[r + nU * c].v * dx[c];
-      t2 += A[r + nU * c].d[0] * dq[c];
-    }
-    double v = -(s * jac * t1) - s * jac * t2;
+    double v = -(s * jac * Adx[r]) - s * jac * Adq[r].d[0];
     if (VISC && r > 0) v += jac * (vL * fL[r] + vR * fR[r]);
     sat[r] = v;
   }
@@ -1880,7 +1877,11 @@ __global__ void __launch_bounds__(kBlock) kInterfaceSatLinearized(BlockView B, P
 // sub-partition's FP64 pipe for the same time whatever the number of active
 // lanes, so the per-entry work is spread over 2 nU lanes (and, with one warp
 // per CTA, over many sub-partitions) instead of running as 2 nU passes in one
-// lane.
+// lane. The lanes evaluate lambda^T A+ dq in closed form on duals; forming A+
+// as a matrix product of duals, dividing both parts of each dual and giving
+// the viscous products to one lane took 313 us where this takes 85 (9216
+// entries of a 3D block), 28 where it takes about 20 (121 entries in 2D, a
+// single wave bound by the chain of one lane).
 template <int ND>
 struct InterfaceLanes {
   static constexpr int perEntry = 2 * (ND + 2);          // (l, side) pairs
@@ -1931,75 +1932,81 @@ __global__ void __launch_bounds__(32) kInterfaceSatAdjoint(BlockView B, Physics 
     jac = B.jac[p];
     sL = B.ff.ifInv[2 * e] * jac;
     sR = -B.ff.ifInv[2 * e + 1] * jac;
-    // This lane's share: the Roe average and one side's incoming Jacobian on
-    // single-derivative dual numbers seeded with d/dq_L[l] give
-    // sum_ij lambda_i (dA_ij/dq_l) dq_j into component l; the l = 0 lanes
-    // also give that side's A^T lambda into every component.
-    D dL[nU], dR[nU], roe[nU];
+    // This lane's share: lambda^T A+(Roe(qL, qR)) dq of one side on
+    // single-derivative dual numbers seeded with d/dq_L[l], whose derivative
+    // goes into component l; the l = 0 lanes also give that side's A^T lambda
+    // into every component.
+    D dL[nU], roe[nU];
     for (int c = 0; c < nU; ++c) {
       dL[c] = D(qL[c]);
       dL[c].d[0] = c == l ? 1.0 : 0.0;
-      dR[c] = D(qR[c]);
     }
-    roeAverage<ND, D>(dL, dR, P.g, roe);
-    D A[nU * nU];
-    incomingJacobian<ND, D>(roe, side == 0 ? mL : mR, P.g, side == 0 ? B.ff.dirL[e] : B.ff.dirR[e], A);
+    roeAverage<ND, D, double>(dL, qR, P.g, roe);
     const double* lam = side == 0 ? lamL : lamR;
     const double sInv = side == 0 ? sL : sR;
-    if (l == 0)
-      for (int r = 0; r < nU; ++r) {
-        double t = A[nU * r].v * lam[0];
-        for (int c = 1; c < nU; ++c) t += A[c + nU * r].v * lam[c];
-        contrib[r] = sInv * t;
-      }
-    double t = 0.0;
-    for (int i = 0; i < nU; ++i) {
-      double w = 0.0;
-      for (int j = 0; j < nU; ++j) w += A[i + nU * j].d[0] * dq[j];
-      t += w * lam[i];
-    }
-    contrib[l] += sInv * t;
+    const Incoming<ND, D> I =
+        incomingState<ND, D>(roe, side == 0 ? mL : mR, P.g, side == 0 ? B.ff.dirL[e] : B.ff.dirR[e]);
+    double grad[nU];
+    const D form = incomingForm<ND, D>(I, lam, dq, grad);
+#pragma unroll
+    for (int c = 0; c < nU; ++c) contrib[c] = (l == 0 ? sInv * grad[c] : 0.0) + (l == c ? sInv * form.d[0] : 0.0);
   }
   for (int c = 0; c < nU; ++c) part[lane][c] = contrib[c];
   __syncwarp();
-  if (!active || k != 0) return;
-  // the entry's lanes' shares summed in lane order, then the viscous terms
+  // the entry's lanes' shares summed in lane order
   double sat[nU];
-  for (int c = 0; c < nU; ++c) {
-    double t = part[lane][c];
-    for (int j = 1; j < G; ++j) t += part[lane + j][c];
-    sat[c] = t;
-  }
-  double u[ND];
-  for (int d = 0; d < ND; ++d) u[d] = fs.prim[p + N * L.u(d)];
+  if (active && k == 0)
+    for (int c = 0; c < nU; ++c) {
+      double t = part[lane][c];
+      for (int j = 1; j < G; ++j) t += part[lane + j][c];
+      sat[c] = t;
+    }
   if (VISC) {
-    double tau[ND * ND], hf[ND];
-    const double v = fs.prim[p + N * L.v()], T = fs.prim[p + N * L.T()];
-    for (int c = 0; c < ND * ND; ++c) tau[c] = fs.tau[p + N * c];
-    for (int d = 0; d < ND; ++d) hf[d] = fs.hf[p + N * d];
-    for (int sd = 0; sd < 2; ++sd) {
-      double y[nU];
-      for (int c = 0; c < nU; ++c) y[c] = 0.0;
-      firstPartialViscousTransposeProduct<ND>(sd == 0 ? mL : mR, u, T, v, P.g, P.powerLawExponent, tau, hf,
-                                              sd == 0 ? lamL : lamR, y);
-      const double sVis = sd == 0 ? -B.ff.ifVis[2 * e] : B.ff.ifVis[2 * e + 1];
-      for (int c = 0; c < nU; ++c) sat[c] += sVis * jac * y[c];
+    // the viscous terms, one product a lane: B1^T lambda of either side (lanes
+    // 0 and 1), then the B2 products of every axis and side
+    __syncwarp();
+    if (active && k < 2 + 2 * ND) {
+      double u[ND];
+      for (int d = 0; d < ND; ++d) u[d] = fs.prim[p + N * L.u(d)];
+      if (k < 2) {
+        double tau[ND * ND], hf[ND], t[nU];
+        const double v = fs.prim[p + N * L.v()], T = fs.prim[p + N * L.T()];
+        for (int c = 0; c < ND * ND; ++c) tau[c] = fs.tau[p + N * c];
+        for (int d = 0; d < ND; ++d) hf[d] = fs.hf[p + N * d];
+        for (int c = 0; c < nU; ++c) t[c] = 0.0;
+        double ms[ND], ls[nU];
+        for (int d = 0; d < ND; ++d) ms[d] = k == 0 ? mL[d] : mR[d];
+        for (int c = 0; c < nU; ++c) ls[c] = k == 0 ? lamL[c] : lamR[c];
+        firstPartialViscousTransposeProduct<ND>(ms, u, T, v, P.g, P.powerLawExponent, tau, hf, ls, t);
+        const double sVis = (k == 0 ? -B.ff.ifVis[2 * e] : B.ff.ifVis[2 * e + 1]) * jac;
+        for (int c = 0; c < nU; ++c) part[lane][c] = sVis * t[c];
+      } else {
+        const int dl = (k - 2) >> 1, sd = (k - 2) & 1;
+        const double mu = fs.prim[p + N * L.mu()], la = fs.prim[p + N * L.la()], kd = fs.prim[p + N * L.k()];
+        double ml[ND], ms[ND], ls[nV], t[nV];
+        for (int d = 0; d < ND; ++d) {
+          ml[d] = B.metrics[p + N * (ND * dl + d)];
+          ms[d] = sd == 0 ? mL[d] : mR[d];
+        }
+        for (int c = 0; c < nV; ++c) {
+          ls[c] = sd == 0 ? lamL[1 + c] : lamR[1 + c];
+          t[c] = 0.0;
+        }
+        secondPartialViscousTransposeProduct<ND>(u, mu, la, kd, jac, ms, ml, ls, t);
+        const double sVis = sd == 0 ? B.ff.ifVis[2 * e] : -B.ff.ifVis[2 * e + 1];
+        for (int c = 0; c < nV; ++c) part[lane][c] = sVis * t[c];
+      }
+    }
+    __syncwarp();
+    if (active && k == 0) {
+      for (int c = 0; c < nU; ++c) sat[c] = (sat[c] + part[lane][c]) + part[lane + 1][c];
+      double* a = B.ff.ifAd + (long long)e * ND * nV;
+      for (int dl = 0; dl < ND; ++dl)
+        for (int c = 0; c < nV; ++c) a[dl * nV + c] = part[lane + 2 + 2 * dl][c] + part[lane + 3 + 2 * dl][c];
     }
   }
-  for (int c = 0; c < nU; ++c) B.ff.visc[(long long)e * nU + c] = sat[c];
-  if (VISC) {
-    const double mu = fs.prim[p + N * L.mu()], la = fs.prim[p + N * L.la()], kd = fs.prim[p + N * L.k()];
-    double* a = B.ff.ifAd + (long long)e * ND * nV;
-    for (int dl = 0; dl < ND; ++dl) {
-      double ml[ND];
-      for (int d = 0; d < ND; ++d) ml[d] = B.metrics[p + N * (ND * dl + d)];
-      double tL[nV], tR[nV];
-      for (int c = 0; c < nV; ++c) tL[c] = tR[c] = 0.0;
-      secondPartialViscousTransposeProduct<ND>(u, mu, la, kd, jac, mL, ml, &lamL[1], tL);
-      secondPartialViscousTransposeProduct<ND>(u, mu, la, kd, jac, mR, ml, &lamR[1], tR);
-      for (int c = 0; c < nV; ++c) a[dl * nV + c] = B.ff.ifVis[2 * e] * tL[c] - B.ff.ifVis[2 * e + 1] * tR[c];
-    }
-  }
+  if (active && k == 0)
+    for (int c = 0; c < nU; ++c) B.ff.visc[(long long)e * nU + c] = sat[c];
 }
 
 // ---------------------------------------------------------------------------
