@@ -47,11 +47,31 @@ constexpr int kBlock = 128;      // pointwise kernels
 constexpr int kMaxTile = 256;    // largest stage-kernel tile
 // Taps of a boundary closure row loaded together by the stage kernels: at
 // 2D sizes the kernels are single waves whose edge tiles end last, so their
-// closure rows issue four loads at a time; 3D kernels and the persistent
-// batched kernel (NC = false, one register budget for all its phases) keep
-// one at a time and the registers that saves.
+// closure rows issue all their loads at once (16 covers every row): 97x81,
+// microseconds per forward / adjoint stage of a run, 26.9 / 35.8 at four
+// loads, 25.1 / 34.5 at six, 24.7 / 32.8 at all; 201^2 39.0 / 57.5 and
+// 38.6 / 57.5. 3D kernels and the persistent batched kernel (NC = false, one
+// register budget for all its phases) keep one at a time and the registers
+// that saves.
 template <int ND, bool NC = true>
-constexpr int kClosureUnroll = (ND == 2 && NC) ? 4 : 1;
+constexpr int kClosureUnroll = (ND == 2 && NC) ? 16 : 1;
+
+// CTAs of kMaxTile threads whose registers an SM must hold, per stage kernel.
+// With the stencils in integers the 3D kernels wait for their taps more than
+// for the FP64 pipe, and more warps hide it until the registers spill.
+// Measured at 128^3, microseconds without a bound -> with (the next values in
+// parentheses): gradient/flux 424 -> 378 at 3 (385 at 4), dissipation 270 ->
+// 264 at 4 (281 at 3, 308 at 5), divergence 476 -> 369 at 7 (396 at 6, 369 at
+// 8), core 775 -> 643 at 4 (662 at 3), diffusion 246 -> 242 at 6 (246 at 7),
+// assembly 309 -> 274 at 5 (275 at 4, 272 at 6). 2D (401x301): divergence
+// 22.6 -> 20.7 at 5 (21.0 at 6), core 41.5 -> 38.7 at 2 (40.1 at 3), gradient/flux
+// 24.6 -> 23.8 at 2 (24.7 at 3); the others as without a bound.
+struct MinBlocks {
+  int gradFlux, dissipation, divergence, core, diffusion, assemble;
+};
+__host__ __device__ constexpr MinBlocks minBlocks(int nD) {
+  return nD == 3 ? MinBlocks{3, 4, 7, 4, 6, 5} : MinBlocks{2, 4, 5, 2, 4, 4};
+}
 
 // Programmatic dependent launch: every kernel lets the next kernel in its
 // stream start launching as soon as all of its own blocks are running, and
@@ -637,7 +657,7 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
 }
 
 template <int ND, bool CURV, bool VISC>
-__global__ void __launch_bounds__(kMaxTile) kGradFlux(BlockView B, Physics P, RunScalars rs, int flags,
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).gradFlux) kGradFlux(BlockView B, Physics P, RunScalars rs, int flags,
                                                       int stage, Tile T) {
   pdlEnter();
   gradFluxPoint<ND, CURV, VISC>(B, P, rs, flags, stage, T, blockIdx.x);
@@ -679,7 +699,7 @@ __device__ __forceinline__ void dissipationPoint(const BlockView& B, const Physi
 }
 
 template <int ND>
-__global__ void __launch_bounds__(kMaxTile) kDissipation(BlockView B, Physics P, const double* __restrict__ src,
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).dissipation) kDissipation(BlockView B, Physics P, const double* __restrict__ src,
                                                          double sign, Tile T) {
   pdlEnter();
   dissipationPoint<ND>(B, P, src, sign, T, blockIdx.x);
@@ -1032,7 +1052,7 @@ __device__ __forceinline__ void forwardDivergencePoint(const BlockView& B, const
 }
 
 template <int ND>
-__global__ void __launch_bounds__(kMaxTile) kForwardDivergence(BlockView B, Physics P, RunScalars rs, int rkStage,
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).divergence) kForwardDivergence(BlockView B, Physics P, RunScalars rs, int rkStage,
                                                                int stage, int controller, Tile T, int lin,
                                                                double linFactor) {
   pdlEnter();
@@ -1312,7 +1332,7 @@ __global__ void __launch_bounds__(2 * kMaxTile) kAdjointCoreSplit(BlockView B, P
 }
 
 template <int ND, bool CURV, bool VISC>
-__global__ void __launch_bounds__(kMaxTile) kAdjointCore(BlockView B, Physics P, RunScalars rs, int stage,
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).core) kAdjointCore(BlockView B, Physics P, RunScalars rs, int stage,
                                                          int fromSlot, Tile T) {
   pdlEnter();
   adjointCorePoint<ND, CURV, VISC>(B, P, rs, stage, fromSlot, T, blockIdx.x);
@@ -1332,7 +1352,7 @@ __device__ __forceinline__ void adjointDiffusionPoint(const BlockView& B, const 
 }
 
 template <int ND>
-__global__ void __launch_bounds__(kMaxTile) kAdjointDiffusion(BlockView B, Tile T) {
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).diffusion) kAdjointDiffusion(BlockView B, Tile T) {
   pdlEnter();
   adjointDiffusionPoint<ND>(B, T, blockIdx.x);
 }
@@ -1345,22 +1365,113 @@ __global__ void __launch_bounds__(kMaxTile) kAdjointDiffusion(BlockView B, Tile 
 // src/AcousticNoiseImpl.f90:208-280) and the RK4 adjoint stage update of
 // that component (src/RK4IntegratorImpl.f90:203-266).
 // ---------------------------------------------------------------------------
+// One thread per point with its components in turn (3D), or one per point and
+// component (2D, whose grids do not fill the GPU per point). The viscous map's
+// shared products and the point's patch data are then formed and read once:
+// 364 -> 315 us at 128^3, bound by the FP64 pipe (79% busy) before.
+__host__ __device__ constexpr bool assemblePerPoint(int nD) { return nD == 3; }
+constexpr int kAllComponents = -1;
+
 template <int ND, bool VISC>
 __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const Physics& P, const RunScalars& rs,
                                                      int rkStage, int stage, double apiFactor, int api, int fromSlot,
-                                                     const Tile& T, int blk) {
+                                                     const Tile& T, int blk, int comp) {
   long long p;
   PointIndex I;
   if (!locate(B, T, blk, p, I)) return;
   constexpr int nU = ND + 2, E = ND + 1;
-  const int c = blockIdx.y;
   const long long N = B.N;
   const PrimLayout L{ND};
   const FwdState fs = forwardState<ND>(B, rs, stage, fromSlot != 0);
-  double r = B.rcore[p + N * c];
   const double v = fs.prim[p + N * L.v()];
+  const double jac = B.jac[p], S = B.sponge[p], cnt = B.tgtCount[p];
+  int entry[3];
+  for (int k = 0; k < 3; ++k) entry[k] = B.ffOfPoint[3 * p + k];
+  const int exc = B.excIdx ? B.excIdx[p] : -1;
+  const int hole = B.iblank[p] == 0;
+  double xE = 0.0;
+  if (VISC) xE = P.g * v * B.t2[p + N * ND];
+  RkCoeffs k{};
+  if (rkStage > 0) k = rkCoeffs(rs);
+  // the stage's cost-target forcing: factor 0 without the adjoint forcing and
+  // at the final stage, else 2, 0.5 or 1 by stage
+  const bool target = !api && nonzero(cnt) && rs.adjointForcingSwitch && !(*rs.step == 1 && stage == 1);
+  double factor = 0.0, F = 0.0;
+  if (target) {
+    factor = stage == 4 ? 2.0 : (stage == 2 ? 0.5 : 1.0);
+    F = -2.0 * B.mt[p] * P.gm1 * (fs.prim[p + N * L.p()] - B.meanP[p]);
+  }
+  // the RHS of component c from r, its core with the viscous map applied
+  auto component = [&](int c, double r) {
+    if (P.dissipation) r += dissipationTerm<ND>(B, P, I, p, c);
+    r = r * jac;
+    for (int i = 0; i < 3; ++i)
+      if (entry[i] >= 0) r += B.ff.visc[(long long)entry[i] * nU + c];
+    const long long kc = p + N * c;
+    const double lam = B.lam[kc];
+    if (nonzero(S)) r += S * lam;
+    if (exc >= 0 && c <= 2) r += B.excF[3LL * exc + c];
+    if (api) {
+      if (nonzero(cnt) && nonzero(apiFactor)) r += apiFactor * B.adjF[kc];
+    } else if (target) {
+      double f;
+      if (c == E) {
+        f = F;
+      } else if (c > 0) {
+        f = -fs.prim[p + N * L.u(c - 1)] * F;
+      } else {
+        double u2 = 0.0;
+        for (int d = 0; d < ND; ++d) {
+          const double ud = fs.prim[p + N * L.u(d)];
+          u2 = d == 0 ? ud * ud : u2 + ud * ud;
+        }
+        f = 0.5 * u2 * F;
+      }
+      for (int i = 0; i < (int)cnt; ++i) r += factor * f;
+    }
+    if (hole) r = 0.0;
+    switch (rkStage) {
+      case 0:
+        B.rhs[kc] = r;
+        break;
+      case 4:
+        B.b1[kc] = lam;
+        B.b2[kc] = lam - k.h6 * r;
+        B.lam[kc] = lam - k.h2 * r;
+        break;
+      case 3:
+        B.b2[kc] = B.b2[kc] - k.h3 * r;
+        B.lam[kc] = B.b1[kc] - k.h2 * r;
+        break;
+      case 2:
+        B.b2[kc] = B.b2[kc] - k.h3 * r;
+        B.lam[kc] = B.b1[kc] - k.dt * r;
+        break;
+      default:
+        B.lam[kc] = B.b2[kc] - k.h6 * r;
+        break;
+    }
+  };
+  if (comp == kAllComponents) {
+    double su = 0.0;
+#pragma unroll
+    for (int c = 1; c <= ND; ++c) {
+      double r = B.rcore[p + N * c];
+      if (VISC) {
+        const double u = fs.prim[p + N * L.u(c - 1)];
+        const double x = v * B.t2[p + N * (c - 1)] - u * xE;
+        r -= x;
+        su = c == 1 ? u * x : su + u * x;
+      }
+      component(c, r);
+    }
+    component(E, VISC ? B.rcore[p + N * E] - xE : B.rcore[p + N * E]);
+    component(0, VISC ? B.rcore[p] + (v * fs.q[p + N * E] * xE + su) : B.rcore[p]);
+    return;
+  }
+  const int c = comp;
+  double r = B.rcore[p + N * c];
   if (VISC) {
-    const double xE = P.g * v * B.t2[p + N * ND];
     if (c == E) {
       r -= xE;
     } else if (c > 0) {
@@ -1375,70 +1486,7 @@ __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const P
       r += v * fs.q[p + N * E] * xE + su;
     }
   }
-  if (P.dissipation) r += dissipationTerm<ND>(B, P, I, p, c);
-  r = r * B.jac[p];
-  for (int k = 0; k < 3; ++k) {
-    const int e = B.ffOfPoint[3 * p + k];
-    if (e >= 0) r += B.ff.visc[(long long)e * nU + c];
-  }
-  const long long kc = p + N * c;
-  const double lam = B.lam[kc];
-  const double S = B.sponge[p];
-  if (nonzero(S)) r += S * lam;
-  if (B.excIdx && c <= 2) {
-    const int e = B.excIdx[p];
-    if (e >= 0) r += B.excF[3LL * e + c];
-  }
-  const double cnt = B.tgtCount[p];
-  if (api) {
-    if (nonzero(cnt) && nonzero(apiFactor)) r += apiFactor * B.adjF[kc];
-  } else if (nonzero(cnt)) {
-    const bool finalStage = (*rs.step == 1 && stage == 1);
-    // factor 0 without the adjoint forcing and at the final stage, else 2, 0.5 or 1 by stage
-    if (rs.adjointForcingSwitch && !finalStage) {
-      const double factor = stage == 4 ? 2.0 : (stage == 2 ? 0.5 : 1.0);
-      const double F = -2.0 * B.mt[p] * P.gm1 * (fs.prim[p + N * L.p()] - B.meanP[p]);
-      double f;
-      if (c == E) {
-        f = F;
-      } else if (c > 0) {
-        f = -fs.prim[p + N * L.u(c - 1)] * F;
-      } else {
-        double u2 = 0.0;
-        for (int d = 0; d < ND; ++d) {
-          const double ud = fs.prim[p + N * L.u(d)];
-          u2 = d == 0 ? ud * ud : u2 + ud * ud;
-        }
-        f = 0.5 * u2 * F;
-      }
-      for (int k = 0; k < (int)cnt; ++k) r += factor * f;
-    }
-  }
-  if (B.iblank[p] == 0) r = 0.0;
-  if (rkStage == 0) {
-    B.rhs[kc] = r;
-    return;
-  }
-  const RkCoeffs k = rkCoeffs(rs);
-  const double h6 = k.h6, h3 = k.h3, h2 = k.h2, dt = k.dt;
-  switch (rkStage) {
-    case 4:
-      B.b1[kc] = lam;
-      B.b2[kc] = lam - h6 * r;
-      B.lam[kc] = lam - h2 * r;
-      break;
-    case 3:
-      B.b2[kc] = B.b2[kc] - h3 * r;
-      B.lam[kc] = B.b1[kc] - h2 * r;
-      break;
-    case 2:
-      B.b2[kc] = B.b2[kc] - h3 * r;
-      B.lam[kc] = B.b1[kc] - dt * r;
-      break;
-    default:
-      B.lam[kc] = B.b2[kc] - h6 * r;
-      break;
-  }
+  component(c, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -1631,11 +1679,12 @@ __global__ void __launch_bounds__(kBlock) kExcitation(BlockView B, ExcPatch X, R
 }
 
 template <int ND, bool VISC>
-__global__ void __launch_bounds__(kMaxTile) kAdjointAssemble(BlockView B, Physics P, RunScalars rs, int rkStage,
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).assemble) kAdjointAssemble(BlockView B, Physics P, RunScalars rs, int rkStage,
                                                              int stage, double apiFactor, int api, int fromSlot,
                                                              Tile T) {
   pdlEnter();
-  adjointAssemblePoint<ND, VISC>(B, P, rs, rkStage, stage, apiFactor, api, fromSlot, T, blockIdx.x);
+  adjointAssemblePoint<ND, VISC>(B, P, rs, rkStage, stage, apiFactor, api, fromSlot, T, blockIdx.x,
+                                 assemblePerPoint(ND) ? kAllComponents : (int)blockIdx.y);
 }
 
 // Adjoint initial condition lambda(T) = factor * adjointForcing(q(T)),
@@ -2691,7 +2740,7 @@ void launchAdjointDiffusion(Context& c, DevBlock& b, cudaStream_t s) {
 void launchAdjointAssemble(Context& c, DevBlock& b, int rkStage, const RunScalars& rs, int stage, double apiFactor,
                            bool api, bool fromSlot, cudaStream_t s) {
   const Tile T = b.tAdjB;
-  const dim3 grid(T.blocks(), c.nU);
+  const dim3 grid(T.blocks(), assemblePerPoint(c.nD) ? 1 : c.nU);
   const int W = T.threads();
   cudaStream_t st = on(c, s);
   MGD_LAUNCH(c);
