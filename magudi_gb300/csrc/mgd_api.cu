@@ -713,7 +713,10 @@ static int autotune(Context& c, DevBlock& b) {
   if (c.nD == 2)
     cands = {{128, 1, 1}, {64, 2, 1}, {32, 4, 1}, {16, 8, 1}, {8, 16, 1},
              {256, 1, 1}, {128, 2, 1}, {64, 4, 1}, {32, 8, 1}, {16, 16, 1}};
-  else
+  // the divergence kernel's CTAs hold every component of their tile
+  const std::vector<std::array<int, 3>> candsDivergence2D = {{64, 1, 1}, {32, 2, 1}, {16, 4, 1}, {8, 8, 1},
+                                                             {128, 1, 1}, {32, 4, 1}, {16, 8, 1}, {8, 16, 1}};
+  if (c.nD == 3)
     cands = {{32, 2, 2}, {32, 4, 1}, {16, 4, 2}, {16, 8, 1}, {8, 8, 2}, {32, 1, 4}, {64, 2, 1},
              {32, 2, 1}, {16, 2, 2}, {8, 4, 4}, {32, 4, 2}};
   RunScalars rs = apiScalars(c);
@@ -744,7 +747,7 @@ static int autotune(Context& c, DevBlock& b) {
       switch (k) {
         case 0: launchGradFlux(c, b, true, false, &rs, 1, false); break;
         case 1: launchDissipation(c, b, b.v.q, 1.0); break;
-        case 2: launchForwardDivergence(c, b, 0, rs, true, false); break;
+        case 2: launchForwardDivergence(c, b, 0, rs, true, false, c.nD == 2); break;
         case 3: launchAdjointCore(c, b, rs, 1, false); break;
         case 4: launchAdjointDiffusion(c, b); break;
         default: launchAdjointAssemble(c, b, 0, rs, 1, 0.0, true, false); break;
@@ -752,18 +755,19 @@ static int autotune(Context& c, DevBlock& b) {
     };
     // the gradient/flux kernel of 2D blocks also has a two-lanes-per-point form
     const int nLaneForms = (k == 0 && c.nD == 2) ? 2 : 1;
-    const int nc = (int)cands.size();
+    const auto& kc = k == 2 && c.nD == 2 ? candsDivergence2D : cands;
+    const int nc = (int)kc.size();
     std::vector<float> ms((size_t)nLaneForms * nc, 1e30f);
     for (int r = 0; r < 20; ++r) launch();  // clocks up before the first timing
     for (int pass = 0; pass < kTunePasses; ++pass)
       for (int lf = 0; lf < nLaneForms; ++lf)
         for (int i = 0; i < nc; ++i) {
-          *slots[k] = makeTile(b, cands[i][0], cands[i][1], cands[i][2]);
+          *slots[k] = makeTile(b, kc[i][0], kc[i][1], kc[i][2]);
           if (k == 0) b.gradLanes = lf + 1;
           ms[(size_t)lf * nc + i] = std::min(ms[(size_t)lf * nc + i], timeIt(launch));
         }
     const int best = (int)(std::min_element(ms.begin(), ms.end()) - ms.begin());
-    *slots[k] = makeTile(b, cands[best % nc][0], cands[best % nc][1], cands[best % nc][2]);
+    *slots[k] = makeTile(b, kc[best % nc][0], kc[best % nc][1], kc[best % nc][2]);
     if (k == 0) b.gradLanes = best / nc + 1;
   }
   c.launches = saved;
@@ -799,7 +803,7 @@ int autotuneTile(Context& c, DevBlock& b, int kernel, const int (*cands)[3], int
     auto run = [&]() {
       if (kernel == BK_GRAD) launchGradFlux(c, b, true, false, &rs, 1, false);
       else if (kernel == BK_DISS) launchDissipation(c, b, b.v.q, 1.0);
-      else launchForwardDivergence(c, b, 0, rs, true, false);
+      else launchForwardDivergence(c, b, 0, rs, true, false, false);
     };
     run();
     cudaEventRecord(e0, c.stream);
@@ -1510,8 +1514,7 @@ void forwardStage(Context& c, DevBlock& b, int rkStage, const RunScalars& rs, bo
   }
   launchGradFlux(c, b, true, false, &rs, stage, store, L.main);
   if (diss || exc) cudaStreamWaitEvent(L.main, L.join, 0);
-  launchForwardDivergence(c, b, rkStage, rs, api, controller, L.main);
-  if (rkStage > 0) launchPrims(c, b, b.v.q, false, nullptr, 0, L.main);
+  launchForwardDivergence(c, b, rkStage, rs, api, controller, rkStage > 0, L.main);
   if (functional) {
     if ((diss || exc) && rkStage >= 1 && rkStage <= 3) {
       // beside the next stage's flux kernel: that stage's side work queues
@@ -1577,8 +1580,7 @@ void regionForwardStage(Context& c, int rkStage, const RunScalars& rs) {
   for (DevBlock& b : c.blocks) launchInterfaceSat(c, b, refs);
   for (DevBlock& b : c.blocks) {
     // actuator patches lie in block 1
-    launchForwardDivergence(c, b, rkStage, rs, true, apiController(c) && &b == &c.blocks[0]);
-    if (rkStage > 0) launchPrims(c, b, b.v.q, false);
+    launchForwardDivergence(c, b, rkStage, rs, true, apiController(c) && &b == &c.blocks[0], rkStage > 0);
   }
 }
 
@@ -2326,8 +2328,7 @@ static void regionRunStage(Context& c, std::vector<DevBlock*>& blocks, std::vect
   cudaStreamWaitEvent(L.main, L.join, 0);
   forEachBlockConcurrently(c, L, [&](int bi, cudaStream_t s) {
     DevBlock& b = *blocks[bi];
-    launchForwardDivergence(c, b, i, rs[bi], false, controller && bi == 0, s);
-    launchPrims(c, b, b.v.q, false, nullptr, 0, s);
+    launchForwardDivergence(c, b, i, rs[bi], false, controller && bi == 0, true, s);
     if (functional) launchFunctional(c, b, rs[bi], i, s);
   });
 }
@@ -3263,8 +3264,9 @@ int mgd_profile_stage_kernels(mgd_ctx* h, int mode, int reps, double* avg_ms, in
   if (mode == MGD_FORWARD) {
     avg_ms[0] = timeIt([&] { launchGradFlux(c, b, true, false, &rs, 2, false); });
     avg_ms[1] = c.phys.dissipation ? timeIt([&] { launchDissipation(c, b, b.v.q, 1.0); }) : 0.0;
-    avg_ms[2] = timeIt([&] { launchForwardDivergence(c, b, 2, rs, false, controller); });
-    avg_ms[3] = timeIt([&] { launchPrims(c, b, b.v.q, false); });
+    avg_ms[2] = timeIt([&] { launchForwardDivergence(c, b, 2, rs, false, controller, c.nD == 2); });
+    // 2D: part of the divergence kernel
+    avg_ms[3] = c.nD == 2 ? 0.0 : timeIt([&] { launchPrims(c, b, b.v.q, false); });
     avg_ms[4] = c.opts.enable_functional ? timeIt([&] { launchFunctional(c, b, rs, 2); }) : 0.0;
   } else {
     if (c.phys.viscous) launchGradFlux(c, b, false, true, &rs, 1, false);

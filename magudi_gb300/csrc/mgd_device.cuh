@@ -104,9 +104,9 @@ __device__ __forceinline__ double closureSum(const double* __restrict__ c, int i
   const double* __restrict__ line = c - i * st;
   if (i < S::depth) {
     const double* __restrict__ row = &g_opLeft[ax.scheme][OP][i * S::width];
-    double s = __ldg(row) * tap<NC>(line);
+    double s = __dmul_rn(__ldg(row), tap<NC>(line));
 #pragma unroll CU
-    for (int k = 1; k < S::width; ++k) s += __ldg(row + k) * tap<NC>(line + k * st);
+    for (int k = 1; k < S::width; ++k) s = fma(__ldg(row + k), tap<NC>(line + k * st), s);
     return s;
   }
   const int m = ax.n - 1 - i;
@@ -115,16 +115,16 @@ __device__ __forceinline__ double closureSum(const double* __restrict__ c, int i
   if (!S::skew && (OP == OP_DISS || OP == OP_DISST) && c_ops.asym[ax.scheme][OP]) {
     // explicit right block, columns left to right
     const double* __restrict__ row = &g_opRight[ax.scheme][OP][m * S::width];
-    double s = __ldg(row) * tap<NC>(end);
+    double s = __dmul_rn(__ldg(row), tap<NC>(end));
 #pragma unroll CU
-    for (int k = 1; k < S::width; ++k) s += __ldg(row + k) * tap<NC>(end + k * st);
+    for (int k = 1; k < S::width; ++k) s = fma(__ldg(row + k), tap<NC>(end + k * st), s);
     return s;
   }
   const double* __restrict__ row = &g_opLeft[ax.scheme][OP][m * S::width];
   // right block = reflection of the left block, negated for skew operators
-  double s = __ldg(row + S::width - 1) * tap<NC>(end);
+  double s = __dmul_rn(__ldg(row + S::width - 1), tap<NC>(end));
 #pragma unroll CU
-  for (int k = 1; k < S::width; ++k) s += __ldg(row + S::width - 1 - k) * tap<NC>(end + k * st);
+  for (int k = 1; k < S::width; ++k) s = fma(__ldg(row + S::width - 1 - k), tap<NC>(end + k * st), s);
   return S::skew ? -s : s;
 }
 

@@ -453,9 +453,10 @@ void launchSolutionLimits(Context& c, DevBlock& b, int blockIndex, const int* st
 // scaled by sign (+1 forward, -1 adjoint).
 void launchDissipation(Context& c, DevBlock& b, const double* src, double sign, cudaStream_t s = 0);
 // Flux divergence, dissipation, 1/det, SATs, sources, then the RK4 forward
-// update of rkStage (or, for rkStage = 0, the RHS into b.v.rhs).
+// update of rkStage (or, for rkStage = 0, the RHS into b.v.rhs); with prims
+// also the primitives of the new state.
 void launchForwardDivergence(Context& c, DevBlock& b, int rkStage, const RunScalars& rs, bool api, bool controller,
-                             cudaStream_t s = 0);
+                             bool prims, cudaStream_t s = 0);
 // Linearized RHS (rkStage 0, into b.v.rhs) or one linearized RK stage of the
 // perturbation in b.v.lam about a forward state: the block's current state
 // (primitives, stress and heat flux current), or with fromSlot the full stage

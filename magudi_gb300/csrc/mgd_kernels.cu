@@ -967,23 +967,25 @@ __device__ __forceinline__ double dissipationTerm(const BlockView& B, const Phys
 // src/RhsHelperImpl.f90:330-351, src/RegionImpl.f90:1968-2023) fused with
 // that component's RK4 forward stage update (src/RK4IntegratorImpl.f90:104-158).
 // ---------------------------------------------------------------------------
-// comp < 0: the component is blockIdx.y (a launch over (tiles, components)).
+// The products and sums are spelled out as multiplications and fused
+// multiply-adds, so that every kernel that holds this function rounds alike.
+// Thread t of tile block blk, component c. The component's new value (its
+// value when rkStage is 0) goes to qNew; false for a thread outside the grid
+// or after a solution-limit violation.
 template <int ND, bool NC = true>
-__device__ __forceinline__ void forwardDivergencePoint(const BlockView& B, const Physics& P, const RunScalars& rs,
+__device__ __forceinline__ bool forwardDivergencePoint(const BlockView& B, const Physics& P, const RunScalars& rs,
                                                        int rkStage, int stage, int controller, const Tile& T,
-                                                       int blk, int lin = 0, double linFactor = 0.0,
-                                                       int comp = -1) {
+                                                       int blk, int t, int c, int lin, double linFactor,
+                                                       long long& p, double& qNew) {
   // after a solution-limit violation in this run the state stays as it is
-  if (rkStage > 0 && rs.limitKey && *rs.limitKey != kNoLimitViolation) return;
-  long long p;
+  if (rkStage > 0 && rs.limitKey && *rs.limitKey != kNoLimitViolation) return false;
   PointIndex I;
-  if (!locate(B, T, blk, p, I)) return;
+  if (!locateAt(B, T, blk, t, p, I)) return false;
   constexpr int nU = ND + 2, E = ND + 1;
-  const int c = comp >= 0 ? comp : (int)blockIdx.y;
   const long long N = B.N;
   double r = -sumOverAxes<ND, OP_D1, NC>(B.fhat + N * c + p, N * nU, I, B);
   if (P.dissipation) r += dissipationTerm<ND, NC>(B, P, I, p, c);
-  r = r * B.jac[p];
+  r = __dmul_rn(r, B.jac[p]);
   for (int k = 0; k < 3; ++k) {
     const int e = B.ffOfPoint[3 * p + k];
     if (e >= 0) r += B.ff.visc[(long long)e * nU + c];
@@ -995,10 +997,10 @@ __device__ __forceinline__ void forwardDivergencePoint(const BlockView& B, const
     // linearized: the sponge acts on the perturbation (q here), the cost
     // target adds its stored adjoint forcing (src/SpongePatchImpl.f90:142-158,
     // src/CostTargetPatchImpl.f90:104-133); no sources, no control
-    if (nonzero(S)) r -= S * q;
-    if (nonzero(linFactor) && nonzero(B.tgtCount[p])) r += linFactor * B.adjF[kc];
+    if (nonzero(S)) r = fma(-S, q, r);
+    if (nonzero(linFactor) && nonzero(B.tgtCount[p])) r = fma(linFactor, B.adjF[kc], r);
   } else if (nonzero(S)) {
-    r -= S * (q - B.qt[kc]);
+    r = fma(-S, q - B.qt[kc], r);
   }
   if (!lin && B.excIdx && (c == 1 || c == 2 || c == E)) {
     const int e = B.excIdx[p];
@@ -1012,43 +1014,46 @@ __device__ __forceinline__ void forwardDivergencePoint(const BlockView& B, const
       const int ai = B.actIdx[p];
       if (ai >= 0) {
         if (rs.apiForcing) {
-          r += B.mc[p] * rs.apiForcing[ai];
+          r = fma(B.mc[p], rs.apiForcing[ai], r);
         } else {
           const long long e = (long long)(rs.nSteps - step) * 4 + (4 - stage);
-          if (e >= 0 && e < rs.nForcingEntries) r += B.mc[p] * rs.forcing[e * rs.P + ai];
+          if (e >= 0 && e < rs.nForcingEntries) r = fma(B.mc[p], rs.forcing[e * rs.P + ai], r);
         }
       }
     }
     if (!lin && B.nSources > 0) {
       const double* amp = rs.amp + ((long long)(step - 1) * 4 + (stage - 1)) * B.nSources;
-      for (int k = 0; k < B.nSources; ++k) r += amp[k] * B.srcG[p + N * k];
+      for (int k = 0; k < B.nSources; ++k) r = fma(amp[k], B.srcG[p + N * k], r);
     }
   }
   if (B.iblank[p] == 0) r = 0.0;
   if (rkStage == 0) {
     B.rhs[kc] = r;
-    return;
+    qNew = q;
+    return true;
   }
   const RkCoeffs k = rkCoeffs(rs);
   const double h6 = k.h6, h3 = k.h3, h2 = k.h2, dt = k.dt;
   switch (rkStage) {
     case 1:
       B.b1[kc] = q;
-      B.b2[kc] = q + h6 * r;
-      B.q[kc] = q + h2 * r;
+      B.b2[kc] = fma(h6, r, q);
+      qNew = fma(h2, r, q);
       break;
     case 2:
-      B.b2[kc] = B.b2[kc] + h3 * r;
-      B.q[kc] = B.b1[kc] + h2 * r;
+      B.b2[kc] = fma(h3, r, B.b2[kc]);
+      qNew = fma(h2, r, B.b1[kc]);
       break;
     case 3:
-      B.b2[kc] = B.b2[kc] + h3 * r;
-      B.q[kc] = B.b1[kc] + dt * r;
+      B.b2[kc] = fma(h3, r, B.b2[kc]);
+      qNew = fma(dt, r, B.b1[kc]);
       break;
     default:
-      B.q[kc] = B.b2[kc] + h6 * r;
+      qNew = fma(h6, r, B.b2[kc]);
       break;
   }
+  B.q[kc] = qNew;
+  return true;
 }
 
 template <int ND>
@@ -1056,7 +1061,35 @@ __global__ void __launch_bounds__(kMaxTile, minBlocks(ND).divergence) kForwardDi
                                                                int stage, int controller, Tile T, int lin,
                                                                double linFactor) {
   pdlEnter();
-  forwardDivergencePoint<ND>(B, P, rs, rkStage, stage, controller, T, blockIdx.x, lin, linFactor);
+  long long p;
+  double q;
+  forwardDivergencePoint<ND>(B, P, rs, rkStage, stage, controller, T, blockIdx.x, threadIdx.x, blockIdx.y, lin,
+                             linFactor, p, q);
+}
+
+// The same with the primitives of the new state, for 2D blocks: a CTA holds
+// every component of its tile (thread = component x tile threads + point), the
+// new values meet in shared memory and the threads of the first component
+// form the primitives. 2D stages are chains of short kernels, and this takes
+// one of three out of the chain.
+__global__ void __maxnreg__(48)
+    kForwardDivergencePrims(BlockView B, Physics P, RunScalars rs, int rkStage, int stage, int controller, Tile T) {
+  pdlEnter();
+  constexpr int nU = 4;
+  __shared__ double share[nU * kMaxTile];
+  const int TT = T.threads();
+  const int c = threadIdx.x / TT, pt = threadIdx.x - c * TT;
+  long long p;
+  double q;
+  const bool ok =
+      forwardDivergencePoint<2>(B, P, rs, rkStage, stage, controller, T, blockIdx.x, pt, c, 0, 0.0, p, q);
+  if (ok) share[c * kMaxTile + pt] = q;
+  __syncthreads();
+  if (!ok || c != 0) return;
+  double state[nU], pr[8];
+  for (int k = 0; k < nU; ++k) state[k] = share[k * kMaxTile + pt];
+  primitives<2>(state, P, pr);
+  for (int k = 0; k < 8; ++k) B.prim[p + B.N * k] = pr[k];
 }
 
 // checkSolutionLimits (src/SolverImpl.f90:189-304) on one point: density and
@@ -2087,7 +2120,10 @@ __global__ void __launch_bounds__(kBatchThreads) kForwardDivergenceBatch(const B
   pdlEnter();
   const int2 m = map[blockIdx.x];
   const BatchEntry& e = E[m.x];
-  forwardDivergencePoint<ND>(e.v, P, e.rs, rkStage, rkStage, e.controller, e.tRhs, m.y, 0, 0.0);
+  long long p;
+  double q;
+  forwardDivergencePoint<ND>(e.v, P, e.rs, rkStage, rkStage, e.controller, e.tRhs, m.y, threadIdx.x, blockIdx.y, 0,
+                             0.0, p, q);
 }
 
 template <int ND>
@@ -2259,7 +2295,10 @@ __global__ void __launch_bounds__(kBatchThreads, persistentMinBlocks(ND))
         const BatchEntry& e = E[w.x];
         RunScalars rs = e.rs;
         rs.step = &sStep;
-        forwardDivergencePoint<ND, false>(e.v, P, rs, stage, stage, e.controller, e.tRhs, w.y, 0, 0.0, w.z);
+        long long p;
+        double q;
+        forwardDivergencePoint<ND, false>(e.v, P, rs, stage, stage, e.controller, e.tRhs, w.y, threadIdx.x, w.z, 0,
+                                          0.0, p, q);
       } else {
         const int2 w = plan.unitsC[u];
         const BlockView& B = E[w.x].v;
@@ -2597,15 +2636,22 @@ void launchDissipation(Context& c, DevBlock& b, const double* src, double sign, 
 }
 
 void launchForwardDivergence(Context& c, DevBlock& b, int rkStage, const RunScalars& rs, bool api, bool controller,
-                             cudaStream_t s) {
+                             bool prims, cudaStream_t s) {
   const int stage = api ? 1 : rkStage;
   const Tile T = b.tRhs;
+  if (prims && c.nD == 2) {
+    MGD_LAUNCH(c);
+    pdl(kForwardDivergencePrims, T.blocks(), c.nU * T.threads(), on(c, s), b.v, c.phys, rs, rkStage, stage, controller,
+        T);
+    return;
+  }
   const dim3 grid(T.blocks(), c.nU);
   MGD_LAUNCH(c);
   if (c.nD == 2)
     pdl(kForwardDivergence<2>, grid, T.threads(), on(c, s), b.v, c.phys, rs, rkStage, stage, controller, T, 0, 0.0);
   else
     pdl(kForwardDivergence<3>, grid, T.threads(), on(c, s), b.v, c.phys, rs, rkStage, stage, controller, T, 0, 0.0);
+  if (prims) launchPrims(c, b, b.v.q, false, nullptr, 0, s);
 }
 
 void launchLinearizedFlux(Context& c, DevBlock& b, const RunScalars& rs, int stage, bool fromSlot, cudaStream_t s) {
