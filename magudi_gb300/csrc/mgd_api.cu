@@ -167,10 +167,11 @@ int mgd_create(const mgd_options* o, mgd_ctx** out) {
   cudaMalloc((void**)&c.dCounters, 8 * sizeof(int));
   const int init[8] = {1, 0, 1, 0, 1, 0, 0, 0};
   cudaMemcpy(c.dCounters, init, sizeof init, cudaMemcpyHostToDevice);
-  cudaMalloc((void**)&c.dApiAmp, MGD_MAX_SOURCES * sizeof(double));
-  cudaMemset(c.dApiAmp, 0, MGD_MAX_SOURCES * sizeof(double));
-  cudaMalloc((void**)&c.dApiTime, sizeof(double));
-  cudaMemset(c.dApiTime, 0, sizeof(double));
+  // the per-call path's stage time follows its source amplitudes
+  if (cudaMalloc((void**)&c.dApiAmp, (MGD_MAX_SOURCES + 1) * sizeof(double)) == cudaSuccess) {
+    cudaMemset(c.dApiAmp, 0, (MGD_MAX_SOURCES + 1) * sizeof(double));
+    c.dApiTime = c.dApiAmp + MGD_MAX_SOURCES;
+  }
   cudaMalloc((void**)&c.dLimitKey, sizeof(unsigned long long));
   cudaMemset(c.dLimitKey, 0xFF, sizeof(unsigned long long));
   cudaMalloc((void**)&c.dKernelError, sizeof(int));
@@ -201,8 +202,8 @@ int mgd_destroy(mgd_ctx* h) {
   cudaFree(c.dLimitKey);
   cudaFree(c.dKernelError);
   cudaFree(c.dCounters); cudaFree(c.dApiAmp); cudaFree(c.dAmp); cudaFree(c.dForcing);
-  cudaFree(c.dApiTime); cudaFree(c.dStageTime); cudaFree(c.dDeltaForcing); cudaFree(c.dApiForcing);
-  cudaFree(c.dGradient); cudaFree(c.dPartials); cudaFree(c.dStageValues);
+  cudaFree(c.dStageTime); cudaFree(c.dDeltaForcing); cudaFree(c.dApiForcing);
+  cudaFree(c.dGradient); cudaFree(c.dPartials); cudaFree(c.dStageValues); cudaFree(c.dQuadrature);
   cudaFree(c.dSnapshots); cudaFree(c.dStageBuf);
   cudaFree(c.dStepDt); cudaFree(c.dDtPartials); cudaFree(c.dTime); cudaFree(c.dNorm);
   if (c.gForward) cudaGraphExecDestroy(c.gForward);
@@ -656,6 +657,7 @@ static void forExtent(const int ext[6], const int gs[3], F f) {
 // per kernel. Results are cached per grid shape and physics flags for the
 // lifetime of the process.
 static RunScalars apiScalars(Context& c);
+static int growDevice(Context& c, double** p, long long* cap, long long need);
 static int setApiTime(Context& c, double time);
 
 struct TuneKey {
@@ -1472,15 +1474,15 @@ static RunScalars apiScalars(Context& c) {
 }
 
 static int setApiTime(Context& c, double time) {
-  double amp[MGD_MAX_SOURCES] = {0};
+  double head[MGD_MAX_SOURCES + 1] = {0};
   const double pi = 4.0 * std::atan(1.0);
   for (size_t s = 0; s < c.sources.size(); ++s) {
     const mgd_acoustic_source& src = c.sources[s];
-    amp[s] = src.amplitude * std::cos(2.0 * pi * src.frequency * time + src.phase);
+    head[s] = src.amplitude * std::cos(2.0 * pi * src.frequency * time + src.phase);
   }
-  CUDA_TRY(c, cudaMemcpyAsync(c.dApiAmp, amp, sizeof amp, cudaMemcpyHostToDevice, c.stream));
+  head[MGD_MAX_SOURCES] = time;
   // pageable source: the copy completes before the call returns
-  CUDA_TRY(c, cudaMemcpyAsync(c.dApiTime, &time, sizeof time, cudaMemcpyHostToDevice, c.stream));
+  CUDA_TRY(c, cudaMemcpyAsync(c.dApiAmp, head, sizeof head, cudaMemcpyHostToDevice, c.stream));
   return 0;
 }
 
@@ -1732,43 +1734,37 @@ static int ensurePartials(Context& c, long long nSlots) {
   return 0;
 }
 
+// Sum over the grid points of the given blocks of the per-call functional's or
+// sensitivity's terms: block partial sums on the device, reduced in a fixed
+// order, one value copied back.
+static int gridSumToHost(Context& c, const std::vector<DevBlock*>& blocks, bool sensitivity, double* value) {
+  long long total = 0;
+  for (const DevBlock* b : blocks) total += quadratureBlocks(*b);
+  if (growDevice(c, &c.dQuadrature, &c.quadratureCapacity, total + 1)) return 1;
+  long long off = 0;
+  for (DevBlock* b : blocks) {
+    launchQuadrature(c, *b, sensitivity, c.dQuadrature + off);
+    off += quadratureBlocks(*b);
+  }
+  launchReducePartials(c, c.dQuadrature, (int)total, (int)total, 1, c.dQuadrature + total);
+  if (checkLaunch(c)) return 1;
+  CUDA_TRY(c, cudaMemcpyAsync(value, c.dQuadrature + total, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c.stream));
+  return 0;
+}
+
 int mgd_compute_functional(mgd_ctx* h, double* value) {
   Context& c = h->c;
   if (requireReady(c)) return 1;
-  double s = 0.0;
-  for (DevBlock& b : c.blocks) {
-    const long long N = b.v.N;
-    std::vector<double> w(N), mt(N), mp(N), pr(N);
-    CUDA_TRY(c, cudaMemcpy(w.data(), b.v.wT, N * sizeof(double), cudaMemcpyDeviceToHost));
-    CUDA_TRY(c, cudaMemcpy(mt.data(), b.v.mt, N * sizeof(double), cudaMemcpyDeviceToHost));
-    CUDA_TRY(c, cudaMemcpy(mp.data(), b.v.meanP, N * sizeof(double), cudaMemcpyDeviceToHost));
-    CUDA_TRY(c, cudaMemcpy(pr.data(), b.v.prim + N * PrimLayout{c.nD}.p(), N * sizeof(double),
-                           cudaMemcpyDeviceToHost));
-    for (long long p = 0; p < N; ++p) {
-      const double F = pr[p] - mp[p];
-      s += w[p] * (F * F * mt[p]);
-    }
-  }
-  *value = s;
-  return 0;
+  std::vector<DevBlock*> blocks;
+  for (DevBlock& b : c.blocks) blocks.push_back(&b);
+  return gridSumToHost(c, blocks, false, value);
 }
 
 int mgd_compute_sensitivity(mgd_ctx* h, double* value) {
   Context& c = h->c;
   if (requireReady(c)) return 1;
-  DevBlock& b = c.blocks[0];
-  const long long N = b.v.N;
-  std::vector<double> w(N), mc(N), lam(N);
-  CUDA_TRY(c, cudaMemcpy(w.data(), b.v.wA, N * sizeof(double), cudaMemcpyDeviceToHost));
-  CUDA_TRY(c, cudaMemcpy(mc.data(), b.v.mc, N * sizeof(double), cudaMemcpyDeviceToHost));
-  CUDA_TRY(c, cudaMemcpy(lam.data(), b.v.lam + N * (c.nD + 1), N * sizeof(double), cudaMemcpyDeviceToHost));
-  double s = 0.0;
-  for (long long p = 0; p < N; ++p) {
-    const double F = lam[p] * mc[p];
-    s += w[p] * (F * F);
-  }
-  *value = s;
-  return 0;
+  return gridSumToHost(c, {&c.blocks[0]}, true, value);
 }
 
 int mgd_rk4_substep(mgd_ctx* h, int mode, double* time, double dt, int stage) {

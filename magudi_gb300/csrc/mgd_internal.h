@@ -309,6 +309,8 @@ struct Context {
   long long partialCapacity = 0;
   double* dStageValues = nullptr;   // per-stage reduced values
   long long stageValueCapacity = 0;
+  double* dQuadrature = nullptr;    // partial sums and the value of a per-call functional or sensitivity
+  long long quadratureCapacity = 0;
   // checkpoints of the last forward run
   int runSteps = 0, saveInterval = 0;
   double runT0 = 0.0;
@@ -502,6 +504,10 @@ void launchAdjointInitial(Context& c, DevBlock& b, double factor);
 void launchStoreAdjointForcing(Context& c, DevBlock& b, bool zero);
 void launchSnapshot(Context& c, DevBlock& b, double* snapshots, int saveInterval, bool initial, cudaStream_t s = 0);
 void launchStepAdvance(Context& c, int delta, cudaStream_t s = 0);
+// Block partial sums (quadratureBlocks of them) of the per-call functional or
+// sensitivity over every grid point.
+int quadratureBlocks(const DevBlock& b);
+void launchQuadrature(Context& c, DevBlock& b, bool sensitivity, double* partials);
 void launchReducePartials(Context& c, const double* partials, int stride, int count, int nSlots, double* out);
 // Constant-CFL step size of the current primitives: with step == null writes
 // the step size to dtOut[0]; otherwise writes dt, dt/6, dt/3, dt/2 to

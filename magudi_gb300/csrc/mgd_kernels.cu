@@ -1071,7 +1071,9 @@ __global__ void __launch_bounds__(kMaxTile, minBlocks(ND).divergence) kForwardDi
 // every component of its tile (thread = component x tile threads + point), the
 // new values meet in shared memory and the threads of the first component
 // form the primitives. 2D stages are chains of short kernels, and this takes
-// one of three out of the chain.
+// one of three out of the chain: 38.6 -> 34.5 us per forward stage at 201^2,
+// 24.7 -> 23.2 at 97x81, 68.9 -> 65.4 at 401x301. 48 registers, so that a
+// single wave of 64-point tiles (256 threads) covers 201^2.
 __global__ void __maxnreg__(48)
     kForwardDivergencePrims(BlockView B, Physics P, RunScalars rs, int rkStage, int stage, int controller, Tile T) {
   pdlEnter();
@@ -1132,6 +1134,30 @@ __device__ __forceinline__ void functionalBlock(const BlockView& B, const RunSca
 __global__ void __launch_bounds__(kBlock) kFunctional(BlockView B, RunScalars rs, int stage, int pressureComp) {
   pdlEnter();
   functionalBlock(B, rs, stage, pressureComp, blockIdx.x);
+}
+
+// The per-call functional (AcousticNoise%compute, src/AcousticNoiseImpl.f90:
+// 123-206) or sensitivity (ThermalActuator%computeSensitivity,
+// src/ThermalActuatorImpl.f90:83-159): block partial sums over every grid
+// point, as the reference's quadrature runs, so that a value that is not a
+// number anywhere on the grid shows. Read on the host, the four fields' copies
+// and the serial sum took about 100 us a call at 201^2.
+__global__ void __launch_bounds__(kBlock) kQuadrature(BlockView B, int sensitivity, int pressureComp, int energyComp,
+                                                      double* __restrict__ partials) {
+  pdlEnter();
+  const long long p = (long long)blockIdx.x * kBlock + threadIdx.x;
+  double v = 0.0;
+  if (p < B.N) {
+    if (sensitivity) {
+      const double F = B.lam[p + B.N * energyComp] * B.mc[p];
+      v = B.wA[p] * (F * F);
+    } else {
+      const double F = B.prim[p + B.N * pressureComp] - B.meanP[p];
+      v = B.wT[p] * (F * F * B.mt[p]);
+    }
+  }
+  const double s = blockSum(v);
+  if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
 // Tangent of the functional at the forward state of (step, stage) along the
@@ -2708,6 +2734,14 @@ void launchLinearized(Context& c, DevBlock& b, int rkStage, const RunScalars& rs
 void launchFunctional(Context& c, DevBlock& b, const RunScalars& rs, int stage, cudaStream_t s) {
   MGD_LAUNCH(c);
   pdl(kFunctional, reductionBlocks(b), kBlock, on(c, s), b.v, rs, stage, PrimLayout{c.nD}.p());
+}
+
+int quadratureBlocks(const DevBlock& b) { return gridFor(b.v.N); }
+
+void launchQuadrature(Context& c, DevBlock& b, bool sensitivity, double* partials) {
+  MGD_LAUNCH(c);
+  pdl(kQuadrature, quadratureBlocks(b), kBlock, c.stream, b.v, (int)sensitivity, PrimLayout{c.nD}.p(), c.nD + 1,
+      partials);
 }
 
 void launchExcitation(Context& c, DevBlock& b, const RunScalars& rs, int stage, bool adjoint, bool fromSlot,
