@@ -444,7 +444,7 @@ int mgd_selftest_pow(const double* x, int n, double e, double* fast, double* ref
 /* Self-test of the interior stencils, which run in integer arithmetic: x
    holds n windows of nine taps (offsets -4..4), out the n results of op 0
    (first derivative), 1 (its adjoint) or 2 (composite dissipation) of the
-   MGD_SBP_* scheme. */
+   MGD_SBP_* scheme, or of op 3, the reciprocal of the centre tap. */
 int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out);
 
 /* Self-test of the bounded wait of the persistent batched kernel (no

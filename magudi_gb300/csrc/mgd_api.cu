@@ -142,6 +142,7 @@ int mgd_create(const mgd_options* o, mgd_ctx** out) {
     }
   }
   P.powerLaw = P.powerLawExponent > 0.0 ? 1 : 0;
+  P.powerLawFixed = fixedExponent(P.powerLawExponent);
   if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess) {
     g_createError = "cudaStreamCreate failed";
     delete h;
@@ -3297,7 +3298,7 @@ int mgd_selftest_fp64_rate(int warps_per_sm, double* lane_ops_per_clock) {
 // Self-test of the table-driven power function used by the viscosity law:
 // evaluates x[i]^e with it (fast) and with CUDA's pow (ref) on the current device.
 int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out) {
-  if (!x || !out || n < 1 || n > (1 << 24) || scheme < 0 || scheme >= kSchemes || op < 0 || op > 2) return 1;
+  if (!x || !out || n < 1 || n > (1 << 24) || scheme < 0 || scheme >= kSchemes || op < 0 || op > 3) return 1;
   double *dx = nullptr, *dout = nullptr;
   cudaError_t e = cudaMalloc((void**)&dx, (size_t)n * 9 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc((void**)&dout, (size_t)n * sizeof(double));

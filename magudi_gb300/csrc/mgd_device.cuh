@@ -879,7 +879,7 @@ __device__ __forceinline__ void adjointPointwise(const double (*w)[ND + 2], cons
         S[x][c] = Pm[x][c] + Pm[c][x];
         X += tau[ND * x + c] * S[x][c];
       }
-    const double NX = P.powerLawExponent * P.g * v / T * X;
+    const double NX = P.powerLawExponent * P.g * v * fixedReciprocal(T) * X;
     S1 += NX;
     y[0] += T * P.invG * NX + v * ug;
     if (boundary(W)) {

@@ -144,6 +144,7 @@ struct Physics {
   double dissipationAmount;
   int viscous, dissipation, composite;
   int powerLaw;  // powerLawExponent > 0: mu follows the power law of T
+  unsigned long long powerLawFixed;  // the exponent in fixed point (fixedExponent), or 0
 };
 
 struct RunScalars {
@@ -580,6 +581,7 @@ constexpr int kMaxExcitationModes = 256;  // modes of one solenoidal-excitation 
 
 // Blocks of the fixed-layout reductions (functional, sensitivity).
 int reductionBlocks(const DevBlock& b);
+unsigned long long fixedExponent(double n);
 void launchPowSelfTest(const double* x, int n, double e, double* fast, double* ref);
 void launchStencilSelfTest(const double* x, int n, int scheme, int op, double* out);
 Tile makeTile(const DevBlock& b, int tx, int ty, int tz);

@@ -29,6 +29,7 @@ namespace mgd {
 
 
 __device__ PowTables g_powTables;
+__device__ FixedPowTables g_fixedPowTables;
 
 static void uploadPowTables() {
   PowTables t;
@@ -41,6 +42,26 @@ static void uploadPowTables() {
   }
   for (int j = 0; j < 64; ++j) t.exp2j[j] = (double)exp2l(j / 64.0L);
   cudaMemcpyToSymbol(g_powTables, &t, sizeof t);
+  static FixedPowTables f;
+  for (int j = 0; j < 512; ++j) {
+    const long double F = 1.0L + (j + 0.5L) / 512.0L;
+    f.g[j] = (uint32_t)std::llround(4294967296.0L / F);
+    f.t[j] = (unsigned long long)std::llround(std::ldexp(-log2l((long double)f.g[j] / 4294967296.0L), 62));
+    f.e[j] = (unsigned long long)std::llround(std::ldexp(exp2l((j + 0.5L) / 512.0L), 62)) << 1;
+  }
+  cudaMemcpyToSymbol(g_fixedPowTables, &f, sizeof f);
+}
+
+// The exponent of fixedPow in Q62, or 0 where x^n stays with fastPowPositive.
+unsigned long long fixedExponent(double n) {
+  return n >= 1.0 / 256.0 && n < 2.0 ? (unsigned long long)std::llround(std::ldexp((long double)n, 62)) : 0ull;
+}
+
+// x^n of the viscosity law.
+__device__ __forceinline__ double powerLaw(double x, double n, unsigned long long nFixed) {
+  double r;
+  if (nFixed && fixedPow(x, nFixed, &g_fixedPowTables, r)) return r;
+  return fastPowPositive(x, n, &g_powTables);
 }
 
 constexpr int kBlock = 128;      // pointwise kernels
@@ -313,7 +334,7 @@ __device__ __forceinline__ double sumOverAxes(const double* x, long long fieldSt
 // computeTransportVariables, src/CNSHelperImpl.f90:3-177).
 template <int ND>
 __device__ __forceinline__ void primitives(const double* q, const Physics& P, double* out /*6+ND*/) {
-  const double v = 1.0 / q[0];
+  const double v = fixedReciprocal(q[0]);
   out[0] = v;
   double u2 = 0.0;
   for (int d = 0; d < ND; ++d) {
@@ -326,7 +347,7 @@ __device__ __forceinline__ void primitives(const double* q, const Physics& P, do
   out[1 + ND] = pr;
   out[2 + ND] = T;
   double mu = P.reInv;
-  if (P.powerLaw) mu = fastPowPositive(P.gm1 * T, P.powerLawExponent, &g_powTables) * P.reInv;
+  if (P.powerLaw) mu = powerLaw(P.gm1 * T, P.powerLawExponent, P.powerLawFixed) * P.reInv;
   out[3 + ND] = mu;
   out[4 + ND] = P.laFactor * mu;
   out[5 + ND] = mu * P.prInv;
@@ -2571,17 +2592,18 @@ __global__ void kFarFieldTargetVisc(BlockView B) {
   }
 }
 
-__global__ void kPowSelfTest(const double* __restrict__ x, int n, double e, double* __restrict__ fast,
-                             double* __restrict__ ref) {
+__global__ void kPowSelfTest(const double* __restrict__ x, int n, double e, unsigned long long eFixed,
+                             double* __restrict__ fast, double* __restrict__ ref) {
   pdlEnter();
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
-  fast[i] = fastPowPositive(x[i], e, &g_powTables);
+  fast[i] = powerLaw(x[i], e, eFixed);
   ref[i] = pow(x[i], e);
 }
 
 // Interior stencils of n windows of nine taps (offsets -4..4): op 0 the first
-// derivative, 1 its adjoint, 2 the composite dissipation.
+// derivative, 1 its adjoint, 2 the composite dissipation; op 3 the reciprocal
+// of the centre tap.
 __global__ void kStencilSelfTest(const double* __restrict__ x, int n, int scheme, int op, double* __restrict__ out) {
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
@@ -2590,7 +2612,8 @@ __global__ void kStencilSelfTest(const double* __restrict__ x, int n, int scheme
   const int idx = 4;
   out[i] = op == 0   ? applyOp<OP_D1>(c, idx, ax)
            : op == 1 ? applyOp<OP_D1ADJ>(c, idx, ax)
-                     : compositeDissipationSum<1, true, 1>(c, &idx, &ax);
+           : op == 2 ? compositeDissipationSum<1, true, 1>(c, &idx, &ax)
+                     : fixedReciprocal(c[0]);
 }
 
 void launchStencilSelfTest(const double* x, int n, int scheme, int op, double* out) {
@@ -2600,7 +2623,7 @@ void launchStencilSelfTest(const double* x, int n, int scheme, int op, double* o
 
 void launchPowSelfTest(const double* x, int n, double e, double* fast, double* ref) {
   uploadOperatorTables();
-  kPowSelfTest<<<(n + kBlock - 1) / kBlock, kBlock>>>(x, n, e, fast, ref);
+  kPowSelfTest<<<(n + kBlock - 1) / kBlock, kBlock>>>(x, n, e, fixedExponent(e), fast, ref);
 }
 
 // ---------------------------------------------------------------------------
