@@ -78,21 +78,26 @@ __device__ __forceinline__ double tap(const double* p) {
   else return __ldca(p);
 }
 
-// Interior stencil of OP over the taps p[j] = x_{j+1}, m[j] = x_{-(j+1)} and
-// the centre x0 (unused by skew operators): the first derivatives in integers
-// where the taps allow it, else in FP64, left to right.
+// Interior stencil of OP in FP64 over the taps p[j] = x_{j+1}, m[j] =
+// x_{-(j+1)} and the centre x0 (unused by skew operators), left to right.
 template <int OP>
-__device__ __forceinline__ double interiorSum(const double* p, const double* m, double x0, int scheme) {
+__device__ __forceinline__ double interiorSumFp64(const double* p, const double* m, double x0, int scheme) {
   using S = OpShape<OP>;
-  if constexpr (OP == OP_D1 || OP == OP_D1ADJ) {
-    double s;
-    if (c_ops.fixed[scheme][OP].valid && fixedSkew(p, m, c_ops.fixed[scheme][OP], s)) return s;
-  }
   const double* __restrict__ cin = c_ops.interior[scheme][OP];
   double s = cin[S::half + 1] * (S::skew ? p[0] - m[0] : p[0] + m[0]);
 #pragma unroll
   for (int j = 2; j <= S::half; ++j) s += cin[S::half + j] * (S::skew ? p[j - 1] - m[j - 1] : p[j - 1] + m[j - 1]);
   return S::skew ? s : s + cin[S::half] * x0;
+}
+
+// Interior stencils of OP of K fields: the first derivatives in integers where
+// the taps allow it.
+template <int OP, int K>
+__device__ __forceinline__ void interiorSums(const double (*p)[4], const double (*m)[4], int scheme, double* out) {
+  static_assert(OP == OP_D1 || OP == OP_D1ADJ, "skew operators");
+  if (c_ops.fixed[scheme][OP].valid && fixedSkew<K>(p, m, c_ops.fixed[scheme][OP], out)) return;
+#pragma unroll
+  for (int k = 0; k < K; ++k) out[k] = interiorSumFp64<OP>(p[k], m[k], 0.0, scheme);
 }
 
 // Boundary closure row of point i (i < depth or i >= n - depth) of a
@@ -171,7 +176,45 @@ __device__ __forceinline__ double applyOp(const double* __restrict__ c, int i, c
       s += cin[S::half + j] * (j < 0 ? m[-j - 1] : (j > 0 ? p[j - 1] : tap<NC>(c)));
     return s;
   }
-  return interiorSum<OP>(p, m, S::skew ? 0.0 : tap<NC>(c), ax.scheme);
+  if constexpr (OP == OP_D1 || OP == OP_D1ADJ) {
+    double s;
+    interiorSums<OP, 1>(&p, &m, ax.scheme, &s);
+    return s;
+  } else {
+    return interiorSumFp64<OP>(p, m, S::skew ? 0.0 : tap<NC>(c), ax.scheme);
+  }
+}
+
+// The first derivative OP of the K fields c + off[k] along one axis, all taps
+// loaded before the first sum (interior) or all fields' closure rows summed
+// side by side: one round of load latency for the axis instead of K.
+template <int OP, int K, bool NC, bool X>
+__device__ __forceinline__ void applyOpFields(const double* __restrict__ c, const long long* off, int i, const Axis& ax,
+                                              double* out) {
+  using S = OpShape<OP>;
+  const long long st = X ? 1 : ax.stride;
+  if (inClosure<OP>(i, ax)) {
+    const bool left = i < S::depth;
+    const double* __restrict__ row = &g_opLeft[ax.scheme][OP][(left ? i : ax.n - 1 - i) * S::width];
+    const double* __restrict__ first = c - i * st + (left ? 0LL : (long long)(ax.n - S::width) * st);
+#pragma unroll
+    for (int w = 0; w < S::width; ++w) {
+      const double r = __ldg(row + (left ? w : S::width - 1 - w));
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double x = tap<NC>(first + off[k] + w * st);
+        out[k] = w == 0 ? __dmul_rn(r, x) : fma(r, x, out[k]);
+      }
+    }
+    if (!left)
+#pragma unroll
+      for (int k = 0; k < K; ++k) out[k] = -out[k];
+    return;
+  }
+  double p[K][4], m[K][4];
+#pragma unroll
+  for (int k = 0; k < K; ++k) interiorTaps<4, NC>(c + off[k], i, st, ax, p[k], m[k]);
+  interiorSums<OP, K>(p, m, ax.scheme, out);
 }
 
 // Composite dissipation sum_d Dc_d x at a point, all axes' interior stencils

@@ -96,31 +96,31 @@ __device__ __forceinline__ double packFixed(long long T, uint32_t r, uint32_t E,
   return __hiloint2double((int)mh, (int)ml);
 }
 
-// A stencil whose largest tap is outside the range of the integer form: 0
-// when every tap is zero (fields at rest), else left to FP64.
-__device__ __forceinline__ bool allZero(const double* t, int n, unsigned long long any, double& out) {
+// Whether n taps are all zero.
+__device__ __forceinline__ bool allZero(const double* t, int n) {
+  unsigned long long any = 0;
 #pragma unroll
   for (int j = 0; j < n; ++j) any |= (unsigned long long)__double_as_longlong(t[j]);
-  out = 0.0;
   return (any << 1) == 0;
 }
 
-// Skew stencil over the taps p[j] = x_{j+1}, m[j] = x_{-(j+1)}. False when the
-// taps are outside the range of the integer form.
-__device__ __forceinline__ bool fixedSkew(const double* p, const double* m, const FixedOp& F, double& out) {
+// Twice the largest high word (sign dropped) of the taps, and whether its
+// exponent lies in the range of the integer form.
+__device__ __forceinline__ uint32_t largestTap(const double* p, const double* m) {
   uint32_t top = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const uint32_t hp = hiWord(p[j]), hm = hiWord(m[j]);
     top = max(top, max(hp + hp, hm + hm));
   }
+  return top;
+}
+__device__ __forceinline__ bool inFixedRange(uint32_t top) { return (top >> 21) - 128u < 1900u; }
+
+// Skew stencil over the taps p[j] = x_{j+1}, m[j] = x_{-(j+1)}, whose largest
+// is in range.
+__device__ __forceinline__ double skewFixed(const double* p, const double* m, uint32_t top, const FixedOp& F) {
   const uint32_t E = top >> 21;
-  if (E - 128u >= 1900u) {
-    double t[8];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) t[j] = p[j], t[4 + j] = m[j];
-    return allZero(t, 8, 0, out);
-  }
   top |= 0x1fffffu;
   const long long d1 = alignTap(p[0], top) - alignTap(m[0], top);
   const long long d2 = alignTap(m[1], top) - alignTap(p[1], top);
@@ -135,7 +135,47 @@ __device__ __forceinline__ bool fixedSkew(const double* p, const double* m, cons
   T += (long long)(int)(d2 >> 32) * F.a[2];
   T += (long long)(int)(d3 >> 32) * F.a[3];
   T += (long long)(int)(d4 >> 32) * F.a[4];
-  out = packFixed<false>(T, (uint32_t)lo, E, F);
+  return packFixed<false>(T, (uint32_t)lo, E, F);
+}
+
+// K skew stencils at once: false when one of them needs FP64. A field at rest
+// (all taps zero) is in range. One branch for all K leaves their sums in one
+// block of code, which the compiler interleaves.
+template <int K>
+__device__ __forceinline__ bool fixedSkew(const double (*p)[4], const double (*m)[4], const FixedOp& F, double* out) {
+  if constexpr (K == 1) {
+    // no value live across the branch
+    const uint32_t t = largestTap(p[0], m[0]);
+    if (!inFixedRange(t)) {
+      out[0] = 0.0;
+      return allZero(p[0], 4) && allZero(m[0], 4);
+    }
+    out[0] = skewFixed(p[0], m[0], t, F);
+    return true;
+  }
+  uint32_t top[K];
+  bool zero[K], ok = true;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    top[k] = largestTap(p[k], m[k]);
+    zero[k] = false;
+    ok = ok && inFixedRange(top[k]);
+  }
+  if (!ok) {
+    ok = true;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (!inFixedRange(top[k])) {
+        zero[k] = allZero(p[k], 4) && allZero(m[k], 4);
+        ok = ok && zero[k];
+      }
+    if (!ok) return false;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const double s = skewFixed(p[k], m[k], top[k], F);
+    out[k] = zero[k] ? 0.0 : s;
+  }
   return true;
 }
 
@@ -153,11 +193,11 @@ __device__ __forceinline__ bool fixedSymmetric(const double (*p)[4], const doubl
       top = max(top, max(hp + hp, hm + hm));
     }
   const uint32_t E = top >> 21;
-  if (E - 128u >= 1900u) {
-    unsigned long long any = (unsigned long long)__double_as_longlong(x0);
-    bool zero = true;
+  if (!inFixedRange(top)) {
+    bool zero = allZero(&x0, 1);
 #pragma unroll
-    for (int d = 0; d < ND; ++d) zero = allZero(p[d], 4, any, out) && allZero(m[d], 4, any, out) && zero;
+    for (int d = 0; d < ND; ++d) zero = allZero(p[d], 4) && allZero(m[d], 4) && zero;
+    out = 0.0;
     return zero;
   }
   top |= 0x1fffffu;

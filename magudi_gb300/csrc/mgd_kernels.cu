@@ -77,6 +77,11 @@ constexpr int kMaxTile = 256;    // largest stage-kernel tile
 template <int ND, bool NC = true>
 constexpr int kClosureUnroll = (ND == 2 && NC) ? 16 : 1;
 
+// Kernels that differentiate several fields at a point take them together in
+// 2D (applyOpFields): its grids leave two or three warps on a sub-partition,
+// and the chain of one field after the other bounds them.
+__host__ __device__ constexpr bool fieldsTogether(int nD, bool nc) { return nD == 2 && nc; }
+
 // CTAs of kMaxTile threads whose registers an SM must hold, per stage kernel.
 // With the stencils in integers the 3D kernels wait for their taps more than
 // for the FP64 pipe, and more warps hide it until the registers spill.
@@ -525,9 +530,10 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
       const int d = lane;
       const int id = d ? I.idx[1] : I.idx[0];
       const Axis ax = d ? B.ax[1] : B.ax[0];
-      const double a0 = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.u(0) + p, id, ax);
-      const double a1 = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.u(1) + p, id, ax);
-      const double aT = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>>(B.prim + N * L.T() + p, id, ax);
+      const long long off[3] = {N * L.u(0), N * L.u(1), N * L.T()};
+      double a[3];
+      applyOpFields<OP_D1, 3, NC, false>(B.prim + p, off, id, ax, a);
+      const double a0 = a[0], a1 = a[1], aT = a[2];
       const unsigned pair = 3u << (threadIdx.x & 30);
       const double b0 = __shfl_xor_sync(pair, a0, 1);
       const double b1 = __shfl_xor_sync(pair, a1, 1);
@@ -538,10 +544,20 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
     } else {
       forEachAxis<ND>([&](auto axis) {
         constexpr int d = decltype(axis)::value;
+        if constexpr (fieldsTogether(ND, NC)) {
+          long long off[ND + 1];
+          double a[ND + 1];
+          for (int c = 0; c < ND; ++c) off[c] = N * L.u(c);
+          off[ND] = N * L.T();
+          applyOpFields<OP_D1, ND + 1, NC, d == 0>(B.prim + p, off, I.idx[d], B.ax[d], a);
+          for (int c = 0; c < ND; ++c) du[c][d] = a[c];
+          dT[d] = a[ND];
+        } else {
 #pragma unroll
-        for (int c = 0; c < ND; ++c)
-          du[c][d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.u(c) + p, I.idx[d], B.ax[d]);
-        dT[d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.T() + p, I.idx[d], B.ax[d]);
+          for (int c = 0; c < ND; ++c)
+            du[c][d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.u(c) + p, I.idx[d], B.ax[d]);
+          dT[d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.T() + p, I.idx[d], B.ax[d]);
+        }
       });
     }
     double gu[ND][ND], gT[ND];
@@ -1294,9 +1310,15 @@ __global__ void __launch_bounds__(kBlock) kAdjointSatVectors(BlockView B, Physic
 template <int ND, int I>
 __device__ __forceinline__ void adjointDerivative(const BlockView& B, long long p, const PointIndex& Ix, double* w) {
   const long long N = B.N;
+  if constexpr (fieldsTogether(ND, true)) {
+    long long off[ND + 2];
+    for (int c = 0; c < ND + 2; ++c) off[c] = N * c;
+    applyOpFields<OP_D1ADJ, ND + 2, true, I == 0>(B.lam + p, off, Ix.idx[I], B.ax[I], w);
+  } else {
 #pragma unroll
-  for (int c = 0; c < ND + 2; ++c)
-    w[c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, I == 0>(B.lam + N * c + p, Ix.idx[I], B.ax[I]);
+    for (int c = 0; c < ND + 2; ++c)
+      w[c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, I == 0>(B.lam + N * c + p, Ix.idx[I], B.ax[I]);
+  }
 }
 
 // The point's core from the adjoint derivatives w along every axis: rcore
@@ -1633,9 +1655,15 @@ __global__ void __launch_bounds__(kMaxTile) kLinearizedFlux(BlockView B, Physics
     jac = B.jac[p];
     forEachAxis<ND>([&](auto axis) {
       constexpr int j = decltype(axis)::value;
+      if constexpr (fieldsTogether(ND, true)) {
+        long long off[nV];
+        for (int c = 0; c < nV; ++c) off[c] = N * c;
+        applyOpFields<OP_D1, nV, true, j == 0>(B.t2 + p, off, I.idx[j], B.ax[j], dt[j]);
+      } else {
 #pragma unroll
-      for (int c = 0; c < nV; ++c)
-        dt[j][c] = applyOp<OP_D1, true, kClosureUnroll<ND>, j == 0>(B.t2 + N * c + p, I.idx[j], B.ax[j]);
+        for (int c = 0; c < nV; ++c)
+          dt[j][c] = applyOp<OP_D1, true, kClosureUnroll<ND>, j == 0>(B.t2 + N * c + p, I.idx[j], B.ax[j]);
+      }
     });
   }
 #pragma unroll
