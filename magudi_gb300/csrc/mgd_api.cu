@@ -714,11 +714,11 @@ static int autotune(Context& c, DevBlock& b) {
   // down. 3D kernels run many waves and also take 64-thread tiles.
   std::vector<std::array<int, 3>> cands;
   if (c.nD == 2)
-    cands = {{128, 1, 1}, {64, 2, 1}, {32, 4, 1}, {16, 8, 1}, {8, 16, 1},
-             {256, 1, 1}, {128, 2, 1}, {64, 4, 1}, {32, 8, 1}, {16, 16, 1}};
-  // the divergence kernel's CTAs hold every component of their tile
-  const std::vector<std::array<int, 3>> candsDivergence2D = {{64, 1, 1}, {32, 2, 1}, {16, 4, 1}, {8, 8, 1},
-                                                             {128, 1, 1}, {32, 4, 1}, {16, 8, 1}, {8, 16, 1}};
+    cands = {{8, 16, 1}, {16, 8, 1}, {32, 4, 1}, {64, 2, 1}, {128, 1, 1},
+             {16, 16, 1}, {32, 8, 1}, {64, 4, 1}, {128, 2, 1}, {256, 1, 1}};
+  // the divergence and (viscous) assembly kernels' CTAs hold every component of their tile
+  const std::vector<std::array<int, 3>> candsAllComponents2D = {{8, 8, 1}, {16, 4, 1}, {32, 2, 1}, {64, 1, 1},
+                                                               {8, 16, 1}, {16, 8, 1}, {32, 4, 1}, {128, 1, 1}};
   if (c.nD == 3)
     cands = {{32, 2, 2}, {32, 4, 1}, {16, 4, 2}, {16, 8, 1}, {8, 8, 2}, {32, 1, 4}, {64, 2, 1},
              {32, 2, 1}, {16, 2, 2}, {8, 4, 4}, {32, 4, 2}};
@@ -752,13 +752,18 @@ static int autotune(Context& c, DevBlock& b) {
         case 1: launchDissipation(c, b, b.v.q, 1.0); break;
         case 2: launchForwardDivergence(c, b, 0, rs, true, false, c.nD == 2); break;
         case 3: launchAdjointCore(c, b, rs, 1, false); break;
-        case 4: launchAdjointDiffusion(c, b); break;
+        case 4:
+          // the separate kernel, which runs of larger blocks use beside the recomputation
+          c.recomputesBeside = true;
+          launchAdjointDiffusion(c, b);
+          c.recomputesBeside = false;
+          break;
         default: launchAdjointAssemble(c, b, 0, rs, 1, 0.0, true, false); break;
       }
     };
     // the gradient/flux kernel of 2D blocks also has a two-lanes-per-point form
     const int nLaneForms = (k == 0 && c.nD == 2) ? 2 : 1;
-    const auto& kc = k == 2 && c.nD == 2 ? candsDivergence2D : cands;
+    const auto& kc = c.nD == 2 && (k == 2 || (k == 5 && assemblyFormsDiffusion(c, b))) ? candsAllComponents2D : cands;
     const int nc = (int)kc.size();
     std::vector<float> ms((size_t)nLaneForms * nc, 1e30f);
     for (int r = 0; r < 20; ++r) launch();  // clocks up before the first timing
@@ -769,7 +774,15 @@ static int autotune(Context& c, DevBlock& b) {
           if (k == 0) b.gradLanes = lf + 1;
           ms[(size_t)lf * nc + i] = std::min(ms[(size_t)lf * nc + i], timeIt(launch));
         }
-    const int best = (int)(std::min_element(ms.begin(), ms.end()) - ms.begin());
+    // Launches back to back end on a grid of about a microsecond, so that 2D
+    // candidates tie; among those within 3% of the fastest the first is taken
+    // (the most compact tile, one thread per point: inside runs, where the
+    // kernels overlap, they are ahead of the others by up to 5%).
+    int best = (int)(std::min_element(ms.begin(), ms.end()) - ms.begin());
+    if (c.nD == 2) {
+      const float limit = 1.03f * ms[best];
+      best = (int)(std::find_if(ms.begin(), ms.end(), [&](float t) { return t <= limit; }) - ms.begin());
+    }
     *slots[k] = makeTile(b, kc[best % nc][0], kc[best % nc][1], kc[best % nc][2]);
     if (k == 0) b.gradLanes = best / nc + 1;
   }
@@ -2559,12 +2572,15 @@ static int regionRunAdjoint(Context& c, double* sensitivity) {
     launchAdjointInitial(c, b, c.opts.adjoint_forcing_switch ? -dtT / 6.0 : 0.0);
   }
   setProgrammaticLaunch(!twoLanes);
+  c.recomputesBeside = twoLanes;
   struct Restore {
+    Context& c;
     ~Restore() {
       setProgrammaticLaunch(true);
       setLaunchPriority(false, 0);
+      c.recomputesBeside = false;
     }
-  } restore;
+  } restore{c};
   // the adjoint is the critical path: the recomputation's kernels launch at
   // the lowest priority and take the SM time the adjoint leaves
   int prioLeast = 0, prioGreatest = 0;
@@ -2774,12 +2790,15 @@ int mgd_run_adjoint(mgd_ctx* h, double* sensitivity) {
   else launchAdjointInitial(c, b, c.opts.adjoint_forcing_switch ? -dtT / 6.0 : 0.0);
   long long nodesRec = 0, nodesAdj = 0;
   setProgrammaticLaunch(!twoLanes);
+  c.recomputesBeside = twoLanes;
   struct Restore {
+    Context& c;
     ~Restore() {
       setProgrammaticLaunch(true);
       setLaunchPriority(false, 0);
+      c.recomputesBeside = false;
     }
-  } restore;
+  } restore{c};
   // The adjoint is the critical path; the recomputation of the next segment
   // has slack (a segment's forward stages take less time than its adjoint
   // stages), so its kernels launch at the lowest priority and take the SM
@@ -3269,7 +3288,8 @@ int mgd_profile_stage_kernels(mgd_ctx* h, int mode, int reps, double* avg_ms, in
     if (c.phys.viscous) launchGradFlux(c, b, false, true, &rs, 1, false);
     avg_ms[0] = timeIt([&] { launchAdjointCore(c, b, rs, 3, false); });
     avg_ms[1] = c.phys.dissipation ? timeIt([&] { launchDissipation(c, b, b.v.lam, -1.0); }) : 0.0;
-    avg_ms[2] = c.phys.viscous ? timeIt([&] { launchAdjointDiffusion(c, b); }) : 0.0;
+    // small 2D blocks: part of the assembly kernel
+    avg_ms[2] = c.phys.viscous && !assemblyFormsDiffusion(c, b) ? timeIt([&] { launchAdjointDiffusion(c, b); }) : 0.0;
     avg_ms[3] = timeIt([&] { launchAdjointAssemble(c, b, 3, rs, 3, 0.0, false, false); });
     avg_ms[4] = timeIt([&] { launchGradientSensitivity(c, b, rs, 3); });
     avg_ms[5] = b.v.ff.n > b.nInterfaceEntries ? timeIt([&] { launchAdjointSatVectors(c, b, rs, 3, false); }) : 0.0;
@@ -3562,7 +3582,8 @@ int mgd_tune_run(mgd_ctx* h, int n_steps, int save_interval, int with_adjoint, d
   if (!rc) rc = timed(&best);
   for (int pass = 0; pass < 2 && !rc; ++pass)
     for (int k = 0; k < 6 && !rc; ++k) {
-      if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous) || (k >= 3 && !with_adjoint)) continue;
+      if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous) || (k >= 3 && !with_adjoint))
+        continue;
       const Tile& cur = slotOf(c.blocks[0], k);
       std::array<int, 3> bestT = {cur.t[0], cur.t[1], cur.t[2]};
       int bestLanes = k == 3 ? c.blocks[0].coreLanes : c.blocks[0].gradLanes;

@@ -314,6 +314,7 @@ struct Context {
   long long quadratureCapacity = 0;
   // checkpoints of the last forward run
   int runSteps = 0, saveInterval = 0;
+  bool recomputesBeside = false;    // an adjoint run's stages are issued beside the recomputation lane
   double runT0 = 0.0;
   std::vector<double> stageTimes;   // time of every forward stage of the run
   double* dSnapshots = nullptr;     // (nSnap) x nU x N per block (single block supported)
@@ -493,6 +494,7 @@ void launchExcitation(Context& c, DevBlock& b, const RunScalars& rs, int stage, 
 // run beside the adjoint core and must complete before the assembly.
 void launchAdjointSatVectors(Context& c, DevBlock& b, const RunScalars& rs, int stage, bool fromSlot,
                              cudaStream_t s = 0);
+bool assemblyFormsDiffusion(const Context& c, const DevBlock& b);
 void launchAdjointDiffusion(Context& c, DevBlock& b, cudaStream_t s = 0);
 // Adjoint: final assembly, SATs, cost-target forcing and the RK4 adjoint update.
 void launchAdjointAssemble(Context& c, DevBlock& b, int rkStage, const RunScalars& rs, int stage, double apiFactor,

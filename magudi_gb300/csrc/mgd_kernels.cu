@@ -661,10 +661,6 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
         }
         continue;
       }
-      if (B.ff.kind[e] != SAT_FAR_FIELD) {
-        wallSatForward<ND, VISC>(B, P, e, p, q, u, B.ff.visc + (long long)e * nU);
-        continue;
-      }
       // sat = -sigma_inv J A+ (q - q_target) + sigma_visc J (F_v - F_v,target) . m
       const double* M = B.ff.M + (long long)e * nU * nU;
       double dqv[nU];
@@ -1481,13 +1477,12 @@ __global__ void __launch_bounds__(kMaxTile, minBlocks(ND).diffusion) kAdjointDif
 __host__ __device__ constexpr bool assemblePerPoint(int nD) { return nD == 3; }
 constexpr int kAllComponents = -1;
 
+// The point's divergence of the viscous diffusion is t2[stride * c].
 template <int ND, bool VISC>
 __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const Physics& P, const RunScalars& rs,
                                                      int rkStage, int stage, double apiFactor, int api, int fromSlot,
-                                                     const Tile& T, int blk, int comp) {
-  long long p;
-  PointIndex I;
-  if (!locate(B, T, blk, p, I)) return;
+                                                     long long p, const PointIndex& I, int comp, const double* t2,
+                                                     long long stride) {
   constexpr int nU = ND + 2, E = ND + 1;
   const long long N = B.N;
   const PrimLayout L{ND};
@@ -1499,7 +1494,7 @@ __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const P
   const int exc = B.excIdx ? B.excIdx[p] : -1;
   const int hole = B.iblank[p] == 0;
   double xE = 0.0;
-  if (VISC) xE = P.g * v * B.t2[p + N * ND];
+  if (VISC) xE = P.g * v * t2[stride * ND];
   RkCoeffs k{};
   if (rkStage > 0) k = rkCoeffs(rs);
   // the stage's cost-target forcing: factor 0 without the adjoint forcing and
@@ -1568,7 +1563,7 @@ __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const P
       double r = B.rcore[p + N * c];
       if (VISC) {
         const double u = fs.prim[p + N * L.u(c - 1)];
-        const double x = v * B.t2[p + N * (c - 1)] - u * xE;
+        const double x = v * t2[stride * (c - 1)] - u * xE;
         r -= x;
         su = c == 1 ? u * x : su + u * x;
       }
@@ -1584,12 +1579,12 @@ __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const P
     if (c == E) {
       r -= xE;
     } else if (c > 0) {
-      r -= v * B.t2[p + N * (c - 1)] - fs.prim[p + N * L.u(c - 1)] * xE;
+      r -= v * t2[stride * (c - 1)] - fs.prim[p + N * L.u(c - 1)] * xE;
     } else {
       double su = 0.0;
       for (int d = 0; d < ND; ++d) {
         const double ud = fs.prim[p + N * L.u(d)];
-        const double xd = v * B.t2[p + N * d] - ud * xE;
+        const double xd = v * t2[stride * d] - ud * xE;
         su = d == 0 ? ud * xd : su + ud * xd;
       }
       r += v * fs.q[p + N * E] * xE + su;
@@ -1798,8 +1793,32 @@ __global__ void __launch_bounds__(kMaxTile, minBlocks(ND).assemble) kAdjointAsse
                                                              int stage, double apiFactor, int api, int fromSlot,
                                                              Tile T) {
   pdlEnter();
-  adjointAssemblePoint<ND, VISC>(B, P, rs, rkStage, stage, apiFactor, api, fromSlot, T, blockIdx.x,
-                                 assemblePerPoint(ND) ? kAllComponents : (int)blockIdx.y);
+  long long p;
+  PointIndex I;
+  if (!locate(B, T, blockIdx.x, p, I)) return;
+  adjointAssemblePoint<ND, VISC>(B, P, rs, rkStage, stage, apiFactor, api, fromSlot, p, I,
+                                 assemblePerPoint(ND) ? kAllComponents : (int)blockIdx.y, B.t2 + p, B.N);
+}
+
+// Diffusion and assembly of viscous 2D blocks in one kernel: a CTA holds every
+// component of its tile (thread = component x tile threads + point), the
+// threads of the first three form the divergence of the viscous diffusion,
+// which all read from shared memory. Takes one of three kernels out of the
+// adjoint stage's chain.
+__global__ void __maxnreg__(56)
+    kAdjointAssembleDiffusion(BlockView B, Physics P, RunScalars rs, int rkStage, int stage, double apiFactor, int api,
+                              int fromSlot, Tile T) {
+  pdlEnter();
+  __shared__ double t2[3 * kMaxTile];
+  const int TT = T.threads();
+  const int c = threadIdx.x / TT, pt = threadIdx.x - c * TT;
+  long long p;
+  PointIndex I;
+  const bool ok = locateAt(B, T, blockIdx.x, pt, p, I);
+  if (ok && c < 3) t2[c * kMaxTile + pt] = sumOverAxes<2, OP_D1ADJ>(B.ad + B.N * c + p, B.N * 3, I, B);
+  __syncthreads();
+  if (!ok) return;
+  adjointAssemblePoint<2, true>(B, P, rs, rkStage, stage, apiFactor, api, fromSlot, p, I, c, t2 + pt, kMaxTile);
 }
 
 // Adjoint initial condition lambda(T) = factor * adjointForcing(q(T)),
@@ -2866,8 +2885,19 @@ void launchAdjointSatVectors(Context& c, DevBlock& b, const RunScalars& rs, int 
   }
 }
 
+// Whether the assembly kernel of a viscous 2D block also forms the viscous
+// diffusion's divergence (kAdjointAssembleDiffusion). A kernel less in the
+// chain pays while the stage leaves the GPU idle: microseconds per adjoint
+// stage of a resident run, separate / fused, 27.3 / 25.0 at 97x81, 50.7 / 42.7
+// at 201^2, 62.2 / 60.0 at 301x261, 72.8 / 74.1 at 361x301. Beside the
+// recomputation lane, which fills that idle time, only the smallest grids
+// gain: 33.4 / 31.8 at 97x81, 56.1 / 57.8 at 201^2, 87.7 / 88.1 at 301x261.
+bool assemblyFormsDiffusion(const Context& c, const DevBlock& b) {
+  return c.nD == 2 && c.phys.viscous && b.v.N <= (c.recomputesBeside ? 16384 : 81920);
+}
+
 void launchAdjointDiffusion(Context& c, DevBlock& b, cudaStream_t s) {
-  if (!c.phys.viscous) return;
+  if (!c.phys.viscous || assemblyFormsDiffusion(c, b)) return;
   const Tile T = b.tAdjD;
   const dim3 grid(T.blocks(), c.nU - 1);
   MGD_LAUNCH(c);
@@ -2877,11 +2907,18 @@ void launchAdjointDiffusion(Context& c, DevBlock& b, cudaStream_t s) {
 
 void launchAdjointAssemble(Context& c, DevBlock& b, int rkStage, const RunScalars& rs, int stage, double apiFactor,
                            bool api, bool fromSlot, cudaStream_t s) {
-  const Tile T = b.tAdjB;
-  const dim3 grid(T.blocks(), assemblePerPoint(c.nD) ? 1 : c.nU);
-  const int W = T.threads();
   cudaStream_t st = on(c, s);
   MGD_LAUNCH(c);
+  if (assemblyFormsDiffusion(c, b)) {
+    const Tile T = b.tAdjB;
+    pdl(kAdjointAssembleDiffusion, T.blocks(), c.nU * T.threads(), st, b.v, c.phys, rs, rkStage, stage, apiFactor, api, fromSlot,
+        T);
+    return;
+  }
+  // the fused form's small tile leaves the separate kernel too few threads a CTA
+  const Tile T = c.nD == 2 && c.phys.viscous && b.tAdjB.threads() < 128 ? b.tAdjD : b.tAdjB;
+  const dim3 grid(T.blocks(), assemblePerPoint(c.nD) ? 1 : c.nU);
+  const int W = T.threads();
 #define AA(ND, VI) \
   pdl(kAdjointAssemble<ND, VI>, grid, W, st, b.v, c.phys, rs, rkStage, stage, apiFactor, api, fromSlot, T)
   if (c.nD == 2) {
