@@ -616,53 +616,24 @@ __host__ __device__ inline void incomingJacobian(const S* cv, const double* metr
     }
 }
 
-// y += (A_i - B1_i)^T w for the inviscid flux Jacobian A along metric m
-// (computeJacobianOfInviscidFlux{2D,3D}, src/CNSHelperImpl.f90:1098-1445) and
-// the first partial viscous Jacobian B1 (computeFirstPartialViscousJacobian,
-// :2412-2601), formed column by column and contracted immediately. P
-// supplies g and the ratios 1/(g-1), (g-2)/(g-1) and 1/g computed once on
-// the host: the per-point divisions by g - 1 and g become multiplications
-// (an FP64 division is about ten FP64 instructions), which changes only
-// rounding.
-template <int ND, bool VISC, class Phys>
-__device__ __forceinline__ void addFluxJacobianTransposeProduct(
-    const double* m, const double* u, double T, double v, const Phys& P, double n,
-    const double* tau, const double* hf, const double* w, double* y) {
+// y += A^T w for the inviscid flux Jacobian A along metric m
+// (computeJacobianOfInviscidFlux{2D,3D}, src/CNSHelperImpl.f90:1098-1445),
+// formed column by column and contracted immediately (wall SATs).
+template <int ND, class Phys>
+__device__ __forceinline__ void addFluxJacobianTransposeProduct(const double* m, const double* u, double T,
+                                                                const Phys& P, const double* w, double* y) {
   const double g = P.g;
-  constexpr int nU = ND + 2, E = ND + 1;
+  constexpr int E = ND + 1;
   double U = m[0] * u[0];
   for (int d = 1; d < ND; ++d) U += m[d] * u[d];
   double u2 = u[0] * u[0];
   for (int d = 1; d < ND; ++d) u2 += u[d] * u[d];
   const double phi2 = 0.5 * (g - 1.0) * u2;
-  // column 0 of A: (0, phi2 m_d - U u_d, U((g-2)/(g-1) phi2 - T))
-  double ct[3] = {0.0, 0.0, 0.0}, t1 = 0.0, uct = 0.0, nTv = 0.0;
-  if (VISC) {
-    for (int a = 0; a < ND; ++a) {
-      double s = m[0] * tau[ND * a];
-      for (int d = 1; d < ND; ++d) s += m[d] * tau[ND * a + d];
-      ct[a] = s;
-    }
-    double cq = m[0] * hf[0];
-    for (int d = 1; d < ND; ++d) cq += m[d] * hf[d];
-    uct = u[0] * ct[0];
-    for (int d = 1; d < ND; ++d) uct += u[d] * ct[d];
-    t1 = uct - cq;
-    nTv = n * g * v / T;
-  }
-  // y_j += sum_i (A(i,j) - B(i,j)) w_i for each column j
   {
-    // j = 0
+    // column 0 of A: (0, phi2 m_d - U u_d, U((g-2)/(g-1) phi2 - T))
     double s = 0.0;
     for (int d = 0; d < ND; ++d) s += (phi2 * m[d] - U * u[d]) * w[1 + d];
     s += U * (P.gm2OverGm1 * phi2 - T) * w[E];
-    if (VISC) {
-      const double t2 = nTv * (phi2 * P.invGm1 - T * P.invG);
-      double sb = 0.0;
-      for (int d = 0; d < ND; ++d) sb += t2 * ct[d] * w[1 + d];
-      sb += (t2 * t1 - v * uct) * w[E];
-      s -= sb;
-    }
     y[0] += s;
   }
   for (int c = 0; c < ND; ++c) {
@@ -672,28 +643,14 @@ __device__ __forceinline__ void addFluxJacobianTransposeProduct(
       s += a * w[1 + d];
     }
     s += ((T + phi2 * P.invGm1) * m[c] - (g - 1.0) * U * u[c]) * w[E];
-    if (VISC) {
-      const double t2 = -nTv * u[c];
-      double sb = 0.0;
-      for (int d = 0; d < ND; ++d) sb += t2 * ct[d] * w[1 + d];
-      sb += (t2 * t1 + v * ct[c]) * w[E];
-      s -= sb;
-    }
     y[1 + c] += s;
   }
   {
     double s = 0.0;
     for (int d = 0; d < ND; ++d) s += (g - 1.0) * m[d] * w[1 + d];
     s += g * U * w[E];
-    if (VISC) {
-      double sb = 0.0;
-      for (int d = 0; d < ND; ++d) sb += nTv * ct[d] * w[1 + d];
-      sb += nTv * t1 * w[E];
-      s -= sb;
-    }
     y[E] += s;
   }
-  (void)nU;
 }
 
 // y += B1^T w alone (first partial viscous Jacobian transpose product), used
@@ -765,16 +722,12 @@ __device__ __forceinline__ void secondPartialViscousTransposeProduct(
   y[ND] += jac * (k * t1) * w[ND];
 }
 
-// Linearized (tangent) flux products, the non-transposed counterparts of the
-// two products above (computeRhsLinearized, src/RhsHelperImpl.f90:655-775).
-// Ax = A(m) x with the rows of computeJacobianOfInviscidFlux{2D,3D}
-// (src/CNSHelperImpl.f90:1098-1445) contracted with x; with VISC also
-// Bx = B1(m) x with the rows of computeFirstPartialViscousJacobian{2D,3D}
-// (:2412-2601). Both are contravariant along the metric row m.
-template <int ND, bool VISC>
-__device__ __forceinline__ void fluxJacobianProduct(const double* m, const double* u, double T, double v, double g,
-                                                    double n, const double* tau, const double* hf, const double* x,
-                                                    double* Ax, double* Bx) {
+// The inviscid linearized flux A(m) x along a metric row (rows of
+// computeJacobianOfInviscidFlux{2D,3D}, src/CNSHelperImpl.f90:1098-1445,
+// contracted with x).
+template <int ND>
+__device__ __forceinline__ void fluxJacobianProduct(const double* m, const double* u, double T, double g,
+                                                    const double* x, double* Ax) {
   constexpr int E = ND + 1;
   double U = m[0] * u[0], u2 = u[0] * u[0], mx = m[0] * x[1], ux = u[0] * x[1];
   for (int d = 1; d < ND; ++d) {
@@ -790,45 +743,109 @@ __device__ __forceinline__ void fluxJacobianProduct(const double* m, const doubl
                 (g - 1.0) * m[d] * x[E];
   Ax[E] = U * ((g - 2.0) / (g - 1.0) * phi2 - T) * x[0] + (T + phi2 / (g - 1.0)) * mx - (g - 1.0) * U * ux +
           g * U * x[E];
-  if (VISC) {
-    double ct[3];
-    for (int a = 0; a < ND; ++a) {
-      double s = m[0] * tau[ND * a];
-      for (int d = 1; d < ND; ++d) s += m[d] * tau[ND * a + d];
-      ct[a] = s;
-    }
-    double cq = m[0] * hf[0], uct = u[0] * ct[0], ctx = ct[0] * x[1];
-    for (int d = 1; d < ND; ++d) {
-      cq += m[d] * hf[d];
-      uct += u[d] * ct[d];
-      ctx += ct[d] * x[1 + d];
-    }
-    const double t1 = uct - cq, nTv = n * g * v / T;
-    const double sg = nTv * ((phi2 / (g - 1.0) - T / g) * x[0] - ux + x[E]);
-    Bx[0] = 0.0;
-    for (int d = 0; d < ND; ++d) Bx[1 + d] = ct[d] * sg;
-    Bx[E] = t1 * sg + v * (ctx - uct * x[0]);
-  }
 }
 
-// y += B2(m1, m2) x (computeSecondPartialViscousJacobian{2D,3D},
-// src/CNSHelperImpl.f90:2636-2757, applied to x); x and y have nD+1 entries.
-template <int ND>
-__device__ __forceinline__ void secondPartialViscousProduct(const double* u, double mu, double la, double k,
-                                                            double jac, const double* m1, const double* m2,
-                                                            const double* x, double* y) {
-  double t1 = m1[0] * m2[0], mx1 = m1[0] * x[0], mx2 = m2[0] * x[0], ux = u[0] * x[0];
-  double m1u = m1[0] * u[0], m2u = m2[0] * u[0];
+// The linearized fluxes of every axis at a point (computeRhsLinearized,
+// src/RhsHelperImpl.f90:655-775): F[i] = A_i x - V[i] and the viscous part
+// V[i] = B1_i x + (0, sum_j B2(m_i, m_j) dt_j), dt[j] the derivative along axis
+// j of (delta u, the temperature perturbation). All are linear in the metric
+// rows, so the Cartesian directions' fluxes are written out first, with
+// D_y = sum_j m_{j,y} dt_j, y_c = x_1+c - u_c x_0, dp the pressure perturbation
+// and H = T + |u|^2/2:
+//   A_x x = (w, u_c w + u_x y_c + [c = x] dp, u_x (dp + x_E - H x_0) + H w), w = x_1+x,
+//   V_x   = (0, t_c = tau_cx sg + J (mu (D_x[c] + D_c[x]) + [c = x] lambda tr D),
+//            (u . tau_x - q_x) sg + v tau_x . y + J (u . S_x + k D_x[E])),
+//   sg = n gamma v / T ((|u|^2/2 - T/gamma) x_0 - u . x_m + x_E),
+// S_x the second half of t. The axes then combine them with their rows.
+template <int ND, bool CURV, bool VISC, class Phys>
+__device__ __forceinline__ void linearizedPointwise(const double* m, const double* u, double T, double v,
+                                                    const Phys& P, const double* tau, const double* hf, double mu,
+                                                    double la, double kd, double jac, const double* x,
+                                                    const double (*dt)[ND + 1], double (*F)[ND + 2],
+                                                    double (*V)[ND + 2]) {
+  constexpr int nU = ND + 2, E = ND + 1;
+  double k = u[0] * u[0], um = u[0] * x[1];
+#pragma unroll
   for (int d = 1; d < ND; ++d) {
-    t1 += m1[d] * m2[d];
-    mx1 += m1[d] * x[d];
-    mx2 += m2[d] * x[d];
-    ux += u[d] * x[d];
-    m1u += m1[d] * u[d];
-    m2u += m2[d] * u[d];
+    k += u[d] * u[d];
+    um += u[d] * x[1 + d];
   }
-  for (int r = 0; r < ND; ++r) y[r] += jac * (mu * t1 * x[r] + mu * m2[r] * mx1 + la * m1[r] * mx2);
-  y[ND] += jac * (mu * t1 * ux + mu * m2u * mx1 + la * m1u * mx2 + k * t1 * x[ND]);
+  k *= 0.5;
+  const double H = T + k, b = k * x[0] - um + x[E];  // dp / (gamma - 1)
+  const double dp = P.gm1 * b, he = dp + x[E] - H * x[0];
+  double y[ND], cF[ND][nU], cV[ND][nU];
+#pragma unroll
+  for (int c = 0; c < ND; ++c) y[c] = x[1 + c] - u[c] * x[0];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const double w = x[1 + d];
+    cF[d][0] = w;
+#pragma unroll
+    for (int c = 0; c < ND; ++c) cF[d][1 + c] = u[c] * w + u[d] * y[c];
+    cF[d][1 + d] += dp;
+    cF[d][E] = u[d] * he + H * w;
+    cV[d][0] = 0.0;
+  }
+  if (VISC) {
+    const double sg = P.powerLawExponent * P.g * v * fixedReciprocal(T) * (b - T * P.invG * x[0]);
+    double D[ND][ND + 1], tr = 0.0;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+#pragma unroll
+      for (int c = 0; c <= ND; ++c) {
+        if (CURV) {
+          double s = m[d] * dt[0][c];
+#pragma unroll
+          for (int j = 1; j < ND; ++j) s += m[ND * j + d] * dt[j][c];
+          D[d][c] = s;
+        } else {
+          D[d][c] = m[ND * d + d] * dt[d][c];
+        }
+      }
+      tr = d ? tr + D[d][d] : D[0][0];
+    }
+    const double jm = jac * mu, jl = jac * la * tr, jk = jac * kd;
+    double S[ND][ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      S[d][d] = 2.0 * jm * D[d][d] + jl;
+#pragma unroll
+      for (int c = d + 1; c < ND; ++c) S[d][c] = S[c][d] = jm * (D[d][c] + D[c][d]);
+    }
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      double e = jk * D[d][ND], t1 = -hf[d], ty = 0.0;
+#pragma unroll
+      for (int c = 0; c < ND; ++c) {
+        const double t = tau[ND * c + d];
+        cV[d][1 + c] = t * sg + S[d][c];
+        t1 += u[c] * t;
+        ty = c ? ty + t * y[c] : t * y[0];
+        e += u[c] * S[d][c];
+      }
+      cV[d][E] = t1 * sg + v * ty + e;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < ND; ++i)
+#pragma unroll
+    for (int c = 0; c < nU; ++c) {
+      double f, g = 0.0;
+      if (CURV) {
+        f = m[ND * i] * cF[0][c];
+        if (VISC) g = m[ND * i] * cV[0][c];
+#pragma unroll
+        for (int d = 1; d < ND; ++d) {
+          f += m[ND * i + d] * cF[d][c];
+          if (VISC) g += m[ND * i + d] * cV[d][c];
+        }
+      } else {
+        f = m[ND * i + i] * cF[i][c];
+        if (VISC) g = m[ND * i + i] * cV[i][c];
+      }
+      F[i][c] = VISC ? f - g : f;
+      V[i][c] = g;
+    }
 }
 
 // The pointwise part of the adjoint core over all directions at once:

@@ -131,6 +131,8 @@ struct Tile {
   int n[3];
   unsigned div[4];
   unsigned long long rcp[4];
+  unsigned rcp32[4];
+  int narrow;  // thread and tile indices times the divisors stay below 2^32: rcp32 divides them exactly
   __host__ __device__ int threads() const { return t[0] * t[1] * t[2]; }
   __host__ __device__ int blocks() const { return n[0] * n[1] * n[2]; }
 };
