@@ -188,11 +188,11 @@ __device__ __forceinline__ double applyOp(const double* __restrict__ c, int i, c
 // The first derivative OP of the K fields c + off[k] along one axis, all taps
 // loaded before the first sum (interior) or all fields' closure rows summed
 // side by side: one round of load latency for the axis instead of K.
-template <int OP, int K, bool NC, bool X>
+template <int OP, int K, bool NC>
 __device__ __forceinline__ void applyOpFields(const double* __restrict__ c, const long long* off, int i, const Axis& ax,
                                               double* out) {
   using S = OpShape<OP>;
-  const long long st = X ? 1 : ax.stride;
+  const long long st = ax.stride;
   if (inClosure<OP>(i, ax)) {
     const bool left = i < S::depth;
     const double* __restrict__ row = &g_opLeft[ax.scheme][OP][(left ? i : ax.n - 1 - i) * S::width];
@@ -215,6 +215,23 @@ __device__ __forceinline__ void applyOpFields(const double* __restrict__ c, cons
 #pragma unroll
   for (int k = 0; k < K; ++k) interiorTaps<4, NC>(c + off[k], i, st, ax, p[k], m[k]);
   interiorSums<OP, K>(p, m, ax.scheme, out);
+}
+
+// The composite dissipation's interior stencils of nAxes axes summed, in
+// integers where the taps allow it (the taps of the other axes are 0).
+template <int ND>
+__device__ __forceinline__ double compositeInteriorSum(const double (*p)[4], const double (*m)[4], double x0, int nAxes,
+                                                       int scheme) {
+  double s;
+  if (c_ops.fixed[scheme][OP_DCOMP].valid && fixedSymmetric<ND>(p, m, x0, nAxes, c_ops.fixed[scheme][OP_DCOMP], s))
+    return s;
+  const double* __restrict__ cin = c_ops.interior[scheme][OP_DCOMP];
+  s = (nAxes * cin[4]) * x0;
+#pragma unroll
+  for (int d = 0; d < ND; ++d)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s += cin[5 + j] * (p[d][j] + m[d][j]);
+  return s;
 }
 
 // Composite dissipation sum_d Dc_d x at a point, all axes' interior stencils
@@ -240,16 +257,7 @@ __device__ __forceinline__ double compositeDissipationSum(const double* __restri
     }
   }
   if (interior == 0) return closure;
-  const int scheme = ax[0].scheme;
-  double s;
-  if (!(c_ops.fixed[scheme][OP_DCOMP].valid && fixedSymmetric<ND>(p, m, x0, interior, c_ops.fixed[scheme][OP_DCOMP], s))) {
-    const double* __restrict__ cin = c_ops.interior[scheme][OP_DCOMP];
-    s = (interior * cin[4]) * x0;
-#pragma unroll
-    for (int d = 0; d < ND; ++d)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s += cin[5 + j] * (p[d][j] + m[d][j]);
-  }
+  const double s = compositeInteriorSum<ND>(p, m, x0, interior, ax[0].scheme);
   return interior == ND ? s : s + closure;
 }
 

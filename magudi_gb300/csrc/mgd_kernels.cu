@@ -86,17 +86,18 @@ __host__ __device__ constexpr bool fieldsTogether(int nD, bool nc) { return nD =
 // With the stencils in integers the 3D kernels wait for their taps more than
 // for the FP64 pipe, and more warps hide it until the registers spill.
 // Measured at 128^3, microseconds without a bound -> with (the next values in
-// parentheses): gradient/flux 424 -> 378 at 3 (385 at 4), dissipation 270 ->
-// 264 at 4 (281 at 3, 308 at 5), divergence 476 -> 369 at 7 (396 at 6, 369 at
-// 8), core 775 -> 643 at 4 (662 at 3), diffusion 246 -> 242 at 6 (246 at 7),
-// assembly 309 -> 274 at 5 (275 at 4, 272 at 6). 2D (401x301): divergence
+// parentheses): gradient/flux 342 at 3 -> 304 at 5 (316 at 4, 298 but 3D jets
+// slower at 6), dissipation 270 -> 264 at 4 (281 at 3, 308 at 5), divergence
+// 476 -> 369 at 7 (396 at 6, 369 at 8), core 538 at 3 -> 540 at 4 with jets 6%
+// faster (544 at 5), diffusion 246 -> 242 at 6 (246 at 7), assembly 309 -> 274
+// at 5 (275 at 4, 272 at 6). 2D (401x301): divergence
 // 22.6 -> 20.7 at 5 (21.0 at 6), core 41.5 -> 38.7 at 2 (40.1 at 3), gradient/flux
 // 24.6 -> 23.8 at 2 (24.7 at 3); the others as without a bound.
 struct MinBlocks {
   int gradFlux, dissipation, divergence, core, diffusion, assemble;
 };
 __host__ __device__ constexpr MinBlocks minBlocks(int nD) {
-  return nD == 3 ? MinBlocks{3, 4, 7, 4, 6, 5} : MinBlocks{2, 4, 5, 2, 4, 4};
+  return nD == 3 ? MinBlocks{5, 4, 7, 4, 6, 5} : MinBlocks{2, 4, 5, 2, 4, 4};
 }
 
 // Programmatic dependent launch: every kernel lets the next kernel in its
@@ -345,6 +346,43 @@ __device__ __forceinline__ double sumOverAxes(const double* x, long long fieldSt
   return s;
 }
 
+// The first derivative OP of K fields along every axis, out[axis][field]; base
+// points at the point, field k lies off(k) beyond it. 2D: a point's fields
+// together (applyOpFields), the axes in a loop that stays one; else one field
+// after the other in a loop per axis. Unrolled further, the kernels wait for
+// their instructions: 2D adjoint stage of a run 57.5 -> 54.6 us at 201^2 and
+// 31.1 -> 29.8 at 97x81 with one copy for both axes; 128^3 core 627 -> 540 and
+// gradient/flux 385 -> 342 with one copy for all fields.
+template <int ND, int OP, int K, bool NC, class Off>
+__device__ __forceinline__ void derivatives(const double* base, Off off, const PointIndex& I, const BlockView& B,
+                                            double (*out)[K]) {
+  if constexpr (fieldsTogether(ND, NC)) {
+    long long o[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) o[k] = off(k);
+#pragma unroll 1
+    for (int d = 0; d < 2; ++d) {
+      double a[K];
+      applyOpFields<OP, K, NC>(base, o, d ? I.idx[1] : I.idx[0], d ? B.ax[1] : B.ax[0], a);
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        // no dynamic register index
+        if (d == 0) out[0][k] = a[k];
+        else out[1][k] = a[k];
+      }
+    }
+  } else {
+    forEachAxis<ND>([&](auto axis) {
+      constexpr int d = decltype(axis)::value;
+      double a[K];
+#pragma unroll 1
+      for (int k = 0; k < K; ++k)
+        a[k] = applyOp<OP, NC, kClosureUnroll<ND, NC>, d == 0>(base + off(k), I.idx[d], B.ax[d]);
+      for (int k = 0; k < K; ++k) out[d][k] = a[k];
+    });
+  }
+}
+
 // Primitive variables of one state (computeDependentVariables +
 // computeTransportVariables, src/CNSHelperImpl.f90:3-177).
 template <int ND>
@@ -542,7 +580,7 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
       const Axis ax = d ? B.ax[1] : B.ax[0];
       const long long off[3] = {N * L.u(0), N * L.u(1), N * L.T()};
       double a[3];
-      applyOpFields<OP_D1, 3, NC, false>(B.prim + p, off, id, ax, a);
+      applyOpFields<OP_D1, 3, NC>(B.prim + p, off, id, ax, a);
       const double a0 = a[0], a1 = a[1], aT = a[2];
       const unsigned pair = 3u << (threadIdx.x & 30);
       const double b0 = __shfl_xor_sync(pair, a0, 1);
@@ -552,23 +590,12 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
       du[1][0] = d ? b1 : a1; du[1][1] = d ? a1 : b1;
       dT[0] = d ? bT : aT; dT[1] = d ? aT : bT;
     } else {
-      forEachAxis<ND>([&](auto axis) {
-        constexpr int d = decltype(axis)::value;
-        if constexpr (fieldsTogether(ND, NC)) {
-          long long off[ND + 1];
-          double a[ND + 1];
-          for (int c = 0; c < ND; ++c) off[c] = N * L.u(c);
-          off[ND] = N * L.T();
-          applyOpFields<OP_D1, ND + 1, NC, d == 0>(B.prim + p, off, I.idx[d], B.ax[d], a);
-          for (int c = 0; c < ND; ++c) du[c][d] = a[c];
-          dT[d] = a[ND];
-        } else {
-#pragma unroll
-          for (int c = 0; c < ND; ++c)
-            du[c][d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.u(c) + p, I.idx[d], B.ax[d]);
-          dT[d] = applyOp<OP_D1, NC, kClosureUnroll<ND, NC>, d == 0>(B.prim + N * L.T() + p, I.idx[d], B.ax[d]);
-        }
-      });
+      double a[ND][ND + 1];
+      derivatives<ND, OP_D1, ND + 1, NC>(B.prim + p, [&](int k) { return N * (k < ND ? L.u(k) : L.T()); }, I, B, a);
+      for (int d = 0; d < ND; ++d) {
+        for (int c = 0; c < ND; ++c) du[c][d] = a[d][c];
+        dT[d] = a[d][ND];
+      }
     }
     double gu[ND][ND], gT[ND];
     for (int x = 0; x < ND; ++x) {
@@ -872,7 +899,6 @@ __global__ void __launch_bounds__(tmadiss::TX* tmadiss::TY)
     for (int k = 0; k <= 2 * H; ++k) loadPlane(k);
     loadHalo(0);
   }
-  const double* __restrict__ cin = c_ops.interior[B.ax[0].scheme][OP_DCOMP];
   const double f = sign * P.dissipationAmount;
   const long long N = B.N;
   // bounded drain of every copy issued up to iteration i (after a wait ran out)
@@ -920,21 +946,14 @@ __global__ void __launch_bounds__(tmadiss::TX* tmadiss::TY)
       return c0[yy * TX + tx];
     };
     auto zAt = [&](int d) { return ring[((i + H + d) % RING) * PLANE + q]; };
-    double sx = cin[H + 1] * (xAt(1) + xAt(-1));
+    double tp[3][H], tm[3][H];
 #pragma unroll
-    for (int j = 2; j <= H; ++j) sx += cin[H + j] * (xAt(j) + xAt(-j));
-    sx = sx + cin[H] * c0[q];
-    double sy = cin[H + 1] * (yAt(1) + yAt(-1));
-#pragma unroll
-    for (int j = 2; j <= H; ++j) sy += cin[H + j] * (yAt(j) + yAt(-j));
-    sy = sy + cin[H] * c0[q];
-    double sz = cin[H + 1] * (zAt(1) + zAt(-1));
-#pragma unroll
-    for (int j = 2; j <= H; ++j) sz += cin[H + j] * (zAt(j) + zAt(-j));
-    sz = sz + cin[H] * c0[q];
-    double s = sx;
-    s += sy;
-    s += sz;
+    for (int j = 1; j <= H; ++j) {
+      tp[0][j - 1] = xAt(j), tm[0][j - 1] = xAt(-j);
+      tp[1][j - 1] = yAt(j), tm[1][j - 1] = yAt(-j);
+      tp[2][j - 1] = zAt(j), tm[2][j - 1] = zAt(-j);
+    }
+    const double s = compositeInteriorSum<3>(tp, tm, c0[q], 3, B.ax[0].scheme);
     const long long p = (x0 + tx) + (long long)nx * ((y0 + ty) + (long long)ny * (z0 + i));
     B.dq[p + N * comp] = f * s;
   }
@@ -1319,21 +1338,6 @@ __global__ void __launch_bounds__(kBlock) kAdjointSatVectors(BlockView B, Physic
   }
 }
 
-// D+_I lambda of every component at a point.
-template <int ND, int I>
-__device__ __forceinline__ void adjointDerivative(const BlockView& B, long long p, const PointIndex& Ix, double* w) {
-  const long long N = B.N;
-  if constexpr (fieldsTogether(ND, true)) {
-    long long off[ND + 2];
-    for (int c = 0; c < ND + 2; ++c) off[c] = N * c;
-    applyOpFields<OP_D1ADJ, ND + 2, true, I == 0>(B.lam + p, off, Ix.idx[I], B.ax[I], w);
-  } else {
-#pragma unroll
-    for (int c = 0; c < ND + 2; ++c)
-      w[c] = applyOp<OP_D1ADJ, true, kClosureUnroll<ND>, I == 0>(B.lam + N * c + p, Ix.idx[I], B.ax[I]);
-  }
-}
-
 // The point's core from the adjoint derivatives w along every axis: rcore
 // and the viscous diffusion ad stored, the far-field viscous penalty and the
 // interface terms included. The SAT vectors of the wall and far-field entries
@@ -1407,10 +1411,8 @@ __device__ __forceinline__ void adjointCorePoint(const BlockView& B, const Physi
   if (!locate(B, T, blk, p, I)) return;
   const FwdState fs = forwardState<ND>(B, rs, stage, fromSlot != 0);
   double w[ND][ND + 2];
-  forEachAxis<ND>([&](auto axis) {
-    constexpr int i = decltype(axis)::value;
-    adjointDerivative<ND, i>(B, p, I, w[i]);
-  });
+  const long long N = B.N;
+  derivatives<ND, OP_D1ADJ, ND + 2, true>(B.lam + p, [&](int k) { return N * k; }, I, B, w);
   adjointCoreFrom<ND, CURV, VISC>(B, P, fs, p, w);
 }
 
@@ -1433,12 +1435,11 @@ __global__ void __launch_bounds__(2 * kMaxTile) kAdjointCoreSplit(BlockView B, P
   const bool ok = locateAt(B, T, blockIdx.x, pt, p, I);
   double w[ND][nU];
   if (ok) {
-    if (dir == 0) {
-      adjointDerivative<ND, 0>(B, p, I, w[0]);
-    } else {
-      adjointDerivative<ND, 1>(B, p, I, w[1]);
-      for (int c = 0; c < nU; ++c) share[c * TT + pt] = w[1][c];
-    }
+    long long off[nU];
+    for (int c = 0; c < nU; ++c) off[c] = B.N * c;
+    applyOpFields<OP_D1ADJ, nU, true>(B.lam + p, off, dir ? I.idx[1] : I.idx[0], dir ? B.ax[1] : B.ax[0], w[0]);
+    if (dir)
+      for (int c = 0; c < nU; ++c) share[c * TT + pt] = w[0][c];
   }
   __syncthreads();
   if (!ok || dir != 0) return;
@@ -1665,18 +1666,7 @@ __global__ void __launch_bounds__(kMaxTile) kLinearizedFlux(BlockView B, Physics
     la = fs.prim[p + N * L.la()];
     kd = fs.prim[p + N * L.k()];
     jac = B.jac[p];
-    forEachAxis<ND>([&](auto axis) {
-      constexpr int j = decltype(axis)::value;
-      if constexpr (fieldsTogether(ND, true)) {
-        long long off[nV];
-        for (int c = 0; c < nV; ++c) off[c] = N * c;
-        applyOpFields<OP_D1, nV, true, j == 0>(B.t2 + p, off, I.idx[j], B.ax[j], dt[j]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < nV; ++c)
-          dt[j][c] = applyOp<OP_D1, true, kClosureUnroll<ND>, j == 0>(B.t2 + N * c + p, I.idx[j], B.ax[j]);
-      }
-    });
+    derivatives<ND, OP_D1, nV, true>(B.t2 + p, [&](int k) { return N * k; }, I, B, dt);
   }
   double F[ND][nU], V[ND][nU];
   linearizedPointwise<ND, CURV, VISC>(m, u, Tm, v, P, tau, hf, mu, la, kd, jac, x, dt, F, V);
