@@ -93,7 +93,7 @@ struct BlockView {
   const double* wA;       // actuator quadrature weight: mask * norm
   const double* tgtCount; // number of cost-target patches holding the point (0 if hole)
   const int* actIdx;      // actuator-patch point index, -1 if none
-  const int* ffOfPoint;   // 3 far-field entry indices per point, -1 if none
+  const int* ffOfPoint;   // up to 3 SAT entry indices per point, the rest -1
   const double* srcG;     // nSources x N: exp(-gaussianFactor r^2), 0 on holes
   int nSources;
   const int* tgtPts;      // points with a cost-target quadrature weight

@@ -6,11 +6,14 @@
 // contravariant fluxes, far-field SAT vector) runs beside kDissipation (one
 // thread per point and component); kForwardDivergence (one thread per point
 // and component) adds the flux divergence, dissipation, SATs and sources and
-// applies the RK update; kPrims refreshes the primitive variables and
-// kFunctional sums the cost functional over the cost-target points.
-// Adjoint RK stage: kAdjointCore (per point) beside kDissipation and
-// kGradientSensitivity; kAdjointDiffusion and kAdjointAssemble (per point and
-// component) finish the adjoint RHS and its RK update.
+// applies the RK update; kPrims refreshes the primitive variables (in 2D
+// kForwardDivergencePrims does both) and kFunctional sums the cost functional
+// over the cost-target points.
+// Adjoint RK stage: kAdjointCore (per point) beside kDissipation,
+// kAdjointSatVectors and kGradientSensitivity; kAdjointDiffusion (per point
+// and component) and kAdjointAssemble (per point in 3D, per point and
+// component in 2D) finish the adjoint RHS and its RK update, in 2D viscous
+// blocks of moderate size in one kernel (kAdjointAssembleDiffusion).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
@@ -665,7 +668,7 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
     }
     for (int s = 0; s < 3 && lane == 0; ++s) {
       const int e = B.ffOfPoint[3 * p + s];
-      if (e < 0) continue;
+      if (e < 0) break;
       const int kind = B.ff.kind[e];
       if (kind != SAT_FAR_FIELD && kind != SAT_INTERFACE) {
         wallSatForward<ND, VISC>(B, P, e, p, q, u, B.ff.visc + (long long)e * nU);
@@ -787,14 +790,18 @@ __global__ void __launch_bounds__(kMaxTile, minBlocks(ND).dissipation) kDissipat
 // axes, with the operands staged in shared memory by the tensor memory
 // accelerator (cp.async.bulk.tensor). A CTA owns a TX x TY column of points
 // (32 x 8 with 16 planes per CTA ran fastest at 128^3 among 32 x 16 and
-// 32 x 8 columns with 8, 16 or 32 planes) and marches through ZC planes of it: a ring of RING planes of the column
+// 32 x 8 columns with 8, 16 or 32 planes, with FP64 sums) and marches through
+// ZC planes of it: a ring of RING planes of the column
 // (z - 4 .. z + 4 and the one being prefetched) feeds the z stencil, and the
 // four halo strips of the current plane (4 points beyond each x and y edge,
 // their coordinates wrapped, so that no copy leaves the grid or overlaps
 // another) feed the x and y stencils. Each tap then reads shared memory
-// instead of global memory. The arithmetic, its order included, is that of
-// dissipationPoint (periodic interior stencil of each axis, x + y + z, times
-// sign x amount). One elected thread issues the copies; every wait on a copy
+// instead of global memory. The arithmetic is that of dissipationPoint: one
+// integer sum over the taps of all axes (compositeInteriorSum), times
+// sign x amount. Bound by the barrier per plane and the integer pipe: 328 us
+// at 128^3 (631 with FP64 sums) against 260 for kDissipation, 65 against 37
+// at 64^3 and 1077 against 857 at 192^3, so it stays a choice of the caller.
+// One elected thread issues the copies; every wait on a copy
 // is bounded, and a wait that runs out sets *err, waits (bounded) for the
 // CTA's copies in flight and leaves.
 // ---------------------------------------------------------------------------
@@ -1031,6 +1038,30 @@ __device__ __forceinline__ double dissipationTerm(const BlockView& B, const Phys
   return sumOverAxes<ND, OP_DISST, NC>(B.dq + N * c + p, N * nU, I, B);
 }
 
+// Whether the point has a SAT entry.
+__device__ __forceinline__ bool anySatEntry(const BlockView& B, long long p) {
+  return B.ffOfPoint[3 * p] >= 0;
+}
+
+// The SAT vectors of component c at the point, one per SAT entry it has.
+// Most points have none, no sponge and no excitation, and their additions as
+// predicated instructions took the FP64 pipe all the same (23 of 66 in the 3D
+// assembly, 6 of 13 per component of the divergence). A loop is not predicated,
+// so the callers branch around it and its neighbours: 128^3 assembly
+// 271 -> 200 us and divergence 375 -> 359-369; a run's forward / adjoint stage at
+// 401x301 59.0 / 120.7 -> 55.7 / 115.1 us, at 201^2 31.5 / 55.0 -> 30.4 / 53.2.
+template <int ND>
+__device__ __forceinline__ double addSatVectors(const BlockView& B, double r, long long p, int c) {
+  constexpr int nU = ND + 2;
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    const int e = B.ffOfPoint[3 * p + k];
+    if (e < 0) break;
+    r += B.ff.visc[(long long)e * nU + c];
+  }
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // Forward RHS of one component (computeRhsForward + Region%computeRhs,
 // src/RhsHelperImpl.f90:330-351, src/RegionImpl.f90:1968-2023) fused with
@@ -1055,26 +1086,24 @@ __device__ __forceinline__ bool forwardDivergencePoint(const BlockView& B, const
   double r = -sumOverAxes<ND, OP_D1, NC>(B.fhat + N * c + p, N * nU, I, B);
   if (P.dissipation) r += dissipationTerm<ND, NC>(B, P, I, p, c);
   r = __dmul_rn(r, B.jac[p]);
-  for (int k = 0; k < 3; ++k) {
-    const int e = B.ffOfPoint[3 * p + k];
-    if (e >= 0) r += B.ff.visc[(long long)e * nU + c];
-  }
   const long long kc = p + N * c;
   const double q = B.q[kc];
   const double S = B.sponge[p];
-  if constexpr (LIN) {
-    // linearized: the sponge acts on the perturbation (q here), the cost
-    // target adds its stored adjoint forcing (src/SpongePatchImpl.f90:142-158,
-    // src/CostTargetPatchImpl.f90:104-133); no sources, no control
-    if (nonzero(S)) r = fma(-S, q, r);
-    if (nonzero(linFactor) && nonzero(B.tgtCount[p])) r = fma(linFactor, B.adjF[kc], r);
-  } else if (nonzero(S)) {
-    r = fma(-S, q - B.qt[kc], r);
-  }
-  if (!LIN && B.excIdx && (c == 1 || c == 2 || c == E)) {
-    const int e = B.excIdx[p];
-    if (e >= 0) r += B.excF[3LL * e + (c == E ? 2 : c - 1)];
-  }
+  const int exc = !LIN && B.excIdx && (c == 1 || c == 2 || c == E) ? B.excIdx[p] : -1;
+  auto patches = [&] {
+    r = addSatVectors<ND>(B, r, p, c);
+    if constexpr (LIN) {
+      // linearized: the sponge acts on the perturbation (q here), the cost
+      // target adds its stored adjoint forcing (src/SpongePatchImpl.f90:142-158,
+      // src/CostTargetPatchImpl.f90:104-133); no sources, no control
+      if (nonzero(S)) r = fma(-S, q, r);
+      if (nonzero(linFactor) && nonzero(B.tgtCount[p])) r = fma(linFactor, B.adjF[kc], r);
+    } else if (nonzero(S)) {
+      r = fma(-S, q - B.qt[kc], r);
+    }
+    if (exc >= 0) r += B.excF[3LL * exc + (c == E ? 2 : c - 1)];
+  };
+  if (LIN || anySatEntry(B, p) || nonzero(S) || exc >= 0) patches();
   if (c == E) {
     const int step = *rs.step;
     // the actuators add the control forcing, or in a tangent run its
@@ -1369,7 +1398,8 @@ __device__ __forceinline__ void adjointCoreFrom(const BlockView& B, const Physic
     bool any = false;
     for (int k = 0; k < 3; ++k) {
       const int e = B.ffOfPoint[3 * p + k];
-      if (e < 0 || B.ff.kind[e] != SAT_FAR_FIELD) continue;
+      if (e < 0) break;
+      if (B.ff.kind[e] != SAT_FAR_FIELD) continue;
       any = true;
       const int nd = B.ff.normalDir[e] - 1;
       const double sv = B.ff.sigVRaw[e];
@@ -1393,7 +1423,8 @@ __device__ __forceinline__ void adjointCoreFrom(const BlockView& B, const Physic
   if (VISC) {
     for (int k = 0; k < 3; ++k) {
       const int e = B.ffOfPoint[3 * p + k];
-      if (e < 0 || B.ff.kind[e] != SAT_INTERFACE) continue;
+      if (e < 0) break;
+      if (B.ff.kind[e] != SAT_INTERFACE) continue;
       const double* a = B.ff.ifAd + (long long)e * ND * nV;
       for (int l = 0; l < ND; ++l)
         for (int c = 0; c < nV; ++c) ad[l][c] += a[l * nV + c];
@@ -1484,7 +1515,8 @@ __global__ void __launch_bounds__(kMaxTile, minBlocks(ND).diffusion) kAdjointDif
 // One thread per point with its components in turn (3D), or one per point and
 // component (2D, whose grids do not fill the GPU per point). The viscous map's
 // shared products and the point's patch data are then formed and read once:
-// 364 -> 315 us at 128^3, bound by the FP64 pipe (79% busy) before.
+// 364 -> 315 us at 128^3, bound by the FP64 pipe (79% busy) before; 271 with
+// the registers of MinBlocks, 200 with the patches branched around.
 __host__ __device__ constexpr bool assemblePerPoint(int nD) { return nD == 3; }
 constexpr int kAllComponents = -1;
 
@@ -1500,9 +1532,8 @@ __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const P
   const FwdState fs = forwardState<ND>(B, rs, stage, fromSlot != 0);
   const double v = fs.prim[p + N * L.v()];
   const double jac = B.jac[p], S = B.sponge[p], cnt = B.tgtCount[p];
-  int entry[3];
-  for (int k = 0; k < 3; ++k) entry[k] = B.ffOfPoint[3 * p + k];
   const int exc = B.excIdx ? B.excIdx[p] : -1;
+  const bool patched = anySatEntry(B, p) || nonzero(S) || exc >= 0;
   const int hole = B.iblank[p] == 0;
   double xE = 0.0;
   if (VISC) xE = P.g * v * t2[stride * ND];
@@ -1520,12 +1551,13 @@ __device__ __forceinline__ void adjointAssemblePoint(const BlockView& B, const P
   auto component = [&](int c, double r) {
     if (P.dissipation) r += dissipationTerm<ND>(B, P, I, p, c);
     r = r * jac;
-    for (int i = 0; i < 3; ++i)
-      if (entry[i] >= 0) r += B.ff.visc[(long long)entry[i] * nU + c];
     const long long kc = p + N * c;
     const double lam = B.lam[kc];
-    if (nonzero(S)) r += S * lam;
-    if (exc >= 0 && c <= 2) r += B.excF[3LL * exc + c];
+    if (patched) {
+      r = addSatVectors<ND>(B, r, p, c);
+      if (nonzero(S)) r += S * lam;
+      if (exc >= 0 && c <= 2) r += B.excF[3LL * exc + c];
+    }
     if (api) {
       if (nonzero(cnt) && nonzero(apiFactor)) r += apiFactor * B.adjF[kc];
     } else if (target) {
