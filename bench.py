@@ -259,27 +259,27 @@ def measured_peaks():
 # needs read or written once; stencil neighbours are re-reads, not counted).
 # bytes: doubles x 8 plus int32 index words x 4. flops: the FP64 operations
 # the kernel executes per point on the 201x201 grid, counted by ncu
-# (2 x DFMA + DADD + DMUL over the launch, divided by the points; the kernels
-# evaluate each term of their operation list once, boundary closure rows
-# included).
+# (2 x DFMA + DADD + DMUL over the launch, divided by the points, boundary
+# closure rows included). Interior stencils run in integers and are not in
+# these counts. The divergence kernel includes the primitives of the new state
+# and the assembly kernel the divergence of the diffusion (the resident form;
+# beside the recomputation lane they are two kernels), so the primitive and
+# diffusion slots of the per-kernel timing are zero.
 KERNEL_UNITS = {
     # q 4, prim (u 2, p, T, mu, la, k) 7, metric diagonal 2, jac 1; writes fhat 8; ffOfPoint 3 ints
-    "forward_gradient_flux": {"bytes": 8 * (4 + 7 + 2 + 1 + 8) + 4 * 3, "flops": 122},
+    "forward_gradient_flux": {"bytes": 8 * (4 + 7 + 2 + 1 + 8) + 4 * 3, "flops": 61},
     # q 4 read, dq 4 written
-    "forward_dissipation": {"bytes": 8 * (4 + 4), "flops": 122},
-    # fhat 8, dq 4, jac 1, q 4, qt 4, sponge 1, srcG 1, b1 4, b2 4 read; b2 4, q 4 written; ffOfPoint 3 + iblank 1 ints
-    "forward_divergence_rk": {"bytes": 8 * (8 + 4 + 1 + 4 + 4 + 1 + 1 + 4 + 4 + 4 + 4) + 4 * 4, "flops": 118},
-    # q 4 read, prim 8 written
-    "forward_primitives": {"bytes": 8 * (4 + 8), "flops": 69},
+    "forward_dissipation": {"bytes": 8 * (4 + 4), "flops": 27},
+    # fhat 8, dq 4, jac 1, q 4, qt 4, sponge 1, srcG 1, b1 4, b2 4 read; b2 4, q 4, prim 8 written; ffOfPoint 3 +
+    # iblank 1 ints
+    "forward_divergence_rk": {"bytes": 8 * (8 + 4 + 1 + 4 + 4 + 1 + 1 + 4 + 4 + 4 + 4 + 8) + 4 * 4, "flops": 68},
     # lambda 4, metric diagonal 2, prim (u 2, v, T, mu, la, k) 7, tau 4, hf 2, jac 1 read; rcore 4, ad 6 written
-    "adjoint_core": {"bytes": 8 * (4 + 2 + 7 + 4 + 2 + 1 + 4 + 6) + 4 * 3, "flops": 469},
+    "adjoint_core": {"bytes": 8 * (4 + 2 + 7 + 4 + 2 + 1 + 4 + 6) + 4 * 3, "flops": 137},
     # lambda 4 read, dq 4 written
-    "adjoint_dissipation": {"bytes": 8 * (4 + 4), "flops": 122},
-    # ad 6 read, t2 3 written
-    "adjoint_diffusion": {"bytes": 8 * (6 + 3), "flops": 84},
-    # rcore 4, prim (v, u 2) 3, q_E 1, t2 3, dq 4, jac 1, lambda 4, sponge 1, tgtCount 1, b1 4, b2 4 read;
+    "adjoint_dissipation": {"bytes": 8 * (4 + 4), "flops": 27},
+    # rcore 4, prim (v, u 2) 3, q_E 1, ad 6, dq 4, jac 1, lambda 4, sponge 1, tgtCount 1, b1 4, b2 4 read;
     # b2 4, lambda 4 written; ffOfPoint 3 + iblank 1 ints
-    "adjoint_assemble_rk": {"bytes": 8 * (4 + 3 + 1 + 3 + 4 + 1 + 4 + 1 + 1 + 4 + 4 + 4 + 4) + 4 * 4, "flops": 47},
+    "adjoint_assemble_rk": {"bytes": 8 * (4 + 3 + 1 + 6 + 4 + 1 + 4 + 1 + 1 + 4 + 4 + 4 + 4) + 4 * 4, "flops": 85},
 }
 # Algorithmic FP64 operations per grid point of the 201x201 monopole RHS:
 # the reference's operation list as the oracle restates it, counted by the
@@ -288,8 +288,8 @@ KERNEL_UNITS = {
 # adjoint_core is the part of computeRhsAdjoint that the adjoint-core kernel
 # performs (adjoint derivatives of lambda, the (A - B1)^T and B2^T products);
 # the GPU kernels evaluate the same terms with fewer operations (the
-# executed counts are in KERNEL_UNITS), so a rate over these counts is the
-# reference-equivalent FP64 rate. forward_gradient_flux is the part of
+# executed counts are in KERNEL_UNITS) and the interior stencils in integers, so
+# a rate over these counts is the reference-equivalent FP64 rate. forward_gradient_flux is the part of
 # updateState after the transport variables (velocity and temperature
 # gradients, stress, heat flux: 95.7) plus the part of computeRhsForward
 # before the derivatives (Cartesian fluxes and their transform: 34.0), which
@@ -299,10 +299,12 @@ ALGORITHMIC_FLOPS = {"forward_rhs": 406.8, "adjoint_rhs": 1073.2, "adjoint_core"
 
 # DRAM bytes (read + write) per launch from an ncu capture of the 201x201
 # gradient workload (dram__bytes_read.sum + dram__bytes_write.sum of one
-# launch of the tuned two-threads-per-point adjoint core, cold L2 between the
-# profiler's passes); kernels not captured are reported as null. The capture
-# and its command are summarised under profiles/.
-MEASURED_TRAFFIC = {"adjoint_core": 7101696 + 0}
+# launch, cold L2 between the profiler's passes; the writes stay in L2);
+# kernels not captured are reported as null. The capture and its command are
+# summarised under profiles/.
+MEASURED_TRAFFIC = {"forward_gradient_flux": 5357056, "forward_dissipation": 1328640,
+                    "forward_divergence_rk": 9990656, "adjoint_core": 6708736, "adjoint_dissipation": 1328640,
+                    "adjoint_assemble_rk": 11493120}
 FORWARD_KERNELS = ["forward_gradient_flux", "forward_dissipation", "forward_divergence_rk", "forward_primitives",
                    "forward_functional"]
 ADJOINT_KERNELS = ["adjoint_core", "adjoint_dissipation", "adjoint_diffusion", "adjoint_assemble_rk",
@@ -645,8 +647,10 @@ def run_ours(args):
                      "hbm": {"achieved_gbs": achieved_gbs, "peak_gbs": peaks["hbm_gbs"],
                              "frac": achieved_gbs / peaks["hbm_gbs"], "bytes_per_point": units["bytes"],
                              "peak_source": peak_kind},
-                     "note": "FP64 path with no tensor-core work: the binding roof is the FP64 pipe; the 201x201 "
-                             "working set stays in L2, so the HBM fraction is not the bound"},
+                     "note": "FP64 path with no tensor-core work; interior stencils run in integers, so the FP64 "
+                             "pipe bounds only the pointwise arithmetic and the closure rows. At 201x201 the kernels "
+                             "are single waves of two to three warps per sub-partition, bound by latency; the working "
+                             "set stays in L2, so the HBM fraction is not the bound"},
     }
     if rank == 0 and world == 1:
         # the same gradient through the per-call entry points (the reference's own

@@ -1,11 +1,14 @@
 // mgd_device.cuh -- device-side building blocks: SBP operator application
 // from constant-memory tables and the pointwise gas dynamics of magudi's
-// CNSHelper (src/CNSHelperImpl.f90), all in FP64.
+// CNSHelper (src/CNSHelperImpl.f90), with FP64 operands and results.
 //
-// Design note: on GB300 FP64 arithmetic runs on a narrow pipe while integer,
-// FP32 and load/store issue slots are plentiful, so these routines minimise
-// FP64 instruction count (no recomputation, algebraic sharing) and leave
-// index arithmetic and loads unoptimised.
+// Design note: on GB300 FP64 arithmetic runs on a narrow pipe (64 cycles a
+// warp instruction and sub-partition). So the interior stencils, the
+// reciprocals and the power law run in integers (mgd_fixed.cuh), and the
+// pointwise algebra shares its products before it forms them. With that, the
+// 3D kernels are near the FP64 and the integer pipe at once, and the code's
+// size and the index arithmetic count too: loops over axes and fields that
+// keep one copy of the stencil code are faster than unrolled ones.
 #pragma once
 
 #include <cstdint>
@@ -876,7 +879,9 @@ __device__ __forceinline__ void linearizedPointwise(const double* m, const doubl
 // energy entries, for ad only, and says whether the point has any.
 // The core is bound by the FP64 pipe (88% busy at 128^3 with each direction's
 // products formed separately: about 440 FP64 instructions a warp, 1735 us);
-// this form takes about 140 (772 us); 201^2 39.6 -> 28.7 us.
+// this form takes about 130 (772 us; 543 with MinBlocks' registers and
+// derivatives()' single copy of the stencil code: FP64 pipe 70% busy before
+// the latter); 201^2 39.6 -> 28.7 us, 20.6 with the latter two.
 template <int ND, bool CURV, bool VISC, class Phys, class Boundary>
 __device__ __forceinline__ void adjointPointwise(const double (*w)[ND + 2], const double* m, const double* u,
                                                  double T, double v, const Phys& P, const double* tau,

@@ -25,7 +25,8 @@
 // kernels, FP64 sums -> integer sums, microseconds a launch: 128^3 periodic,
 // composite dissipation 623 -> 270 (74% of the integer pipe), gradient/flux
 // 681 -> 425, divergence 701 -> 476, adjoint diffusion 404 -> 246; 201^2,
-// 12.3 -> 8.2, 20.5 -> 16.4, 16.4 -> 12.4 and 10.4 -> 8.3.
+// 12.3 -> 8.2, 20.5 -> 16.4, 16.4 -> 12.4 and 10.4 -> 8.3. (By this change
+// alone; the kernels' comments have what followed.)
 #pragma once
 
 #include <cstdint>
