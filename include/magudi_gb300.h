@@ -437,8 +437,9 @@ int mgd_control_zaxpy(mgd_ctx* ctx, double a, int accumulate);
 int mgd_profile_stage_kernels(mgd_ctx* ctx, int mode, int reps, double* avg_ms, int* n_kernels);
 
 /* Self-test (no reference counterpart): evaluates x[i]^e on the current
- * device with the library's table-driven power function (fast) and with
- * CUDA's pow (ref), for checking the viscosity law's error bound. */
+ * device with the library's power function (fast: fixed point, FP64 beyond its
+ * range) and with CUDA's pow (ref), for checking the viscosity law's error
+ * bound. */
 int mgd_selftest_pow(const double* x, int n, double e, double* fast, double* ref);
 
 /* Self-test of the interior stencils, which run in integer arithmetic: x
@@ -446,6 +447,13 @@ int mgd_selftest_pow(const double* x, int n, double e, double* fast, double* ref
    (first derivative), 1 (its adjoint) or 2 (composite dissipation) of the
    MGD_SBP_* scheme, or of op 3, the reciprocal of the centre tap. */
 int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out);
+
+/* The same for stencils that are formed together: form 0 the first derivative
+   of three fields (x: n groups of three windows of nine taps, out: 3 n), 1 its
+   adjoint of four fields (n groups of four, 4 n), 2 and 3 the composite
+   dissipation summed over two and three axes (n boxes of 9^2 or 9^3 points, x
+   fastest, out: its n values at the centres). */
+int mgd_selftest_stencil_group(const double* x, int n, int scheme, int form, double* out);
 
 /* Self-test of the bounded wait of the persistent batched kernel (no
  * reference counterpart), used as a grid barrier: a cooperative launch of

@@ -3315,24 +3315,38 @@ int mgd_selftest_fp64_rate(int warps_per_sm, double* lane_ops_per_clock) {
   return selftestFp64Rate(warps_per_sm, lane_ops_per_clock) ? 1 : 0;
 }
 
-// Self-test of the table-driven power function used by the viscosity law:
-// evaluates x[i]^e with it (fast) and with CUDA's pow (ref) on the current device.
-int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out) {
-  if (!x || !out || n < 1 || n > (1 << 24) || scheme < 0 || scheme >= kSchemes || op < 0 || op > 3) return 1;
+// launch(x, out) on device copies of nIn doubles, nOut results read back.
+template <class Launch>
+static int selftestOnDevice(const double* x, size_t nIn, double* out, size_t nOut, Launch launch) {
   double *dx = nullptr, *dout = nullptr;
-  cudaError_t e = cudaMalloc((void**)&dx, (size_t)n * 9 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&dout, (size_t)n * sizeof(double));
-  if (e == cudaSuccess) e = cudaMemcpy(dx, x, (size_t)n * 9 * sizeof(double), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMalloc((void**)&dx, nIn * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&dout, nOut * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemcpy(dx, x, nIn * sizeof(double), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
-    launchStencilSelfTest(dx, n, scheme, op, dout);
+    launch(dx, dout);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(out, dout, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(out, dout, nOut * sizeof(double), cudaMemcpyDeviceToHost);
   cudaFree(dx);
   cudaFree(dout);
   return e == cudaSuccess ? 0 : 1;
 }
 
+int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out) {
+  if (!x || !out || n < 1 || n > (1 << 24) || scheme < 0 || scheme >= kSchemes || op < 0 || op > 3) return 1;
+  return selftestOnDevice(x, (size_t)n * 9, out, (size_t)n,
+                          [&](double* dx, double* dout) { launchStencilSelfTest(dx, n, scheme, op, dout); });
+}
+
+int mgd_selftest_stencil_group(const double* x, int n, int scheme, int form, double* out) {
+  if (!x || !out || n < 1 || n > (1 << 16) || scheme < 0 || scheme >= kSchemes || form < 0 || form > 3) return 1;
+  static const int in[4] = {3 * 9, 4 * 9, 81, 729}, results[4] = {3, 4, 1, 1};
+  return selftestOnDevice(x, (size_t)n * in[form], out, (size_t)n * results[form],
+                          [&](double* dx, double* dout) { launchStencilGroupSelfTest(dx, n, scheme, form, dout); });
+}
+
+// The power function of the viscosity law (fixed point, FP64 beyond its range)
+// as x[i]^e (fast) and CUDA's pow (ref) on the current device.
 int mgd_selftest_pow(const double* x, int n, double e, double* fast, double* ref) {
   if (n <= 0) return 0;
   double *dx = nullptr, *df = nullptr, *dr = nullptr;

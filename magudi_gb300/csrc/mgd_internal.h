@@ -588,6 +588,7 @@ int reductionBlocks(const DevBlock& b);
 unsigned long long fixedExponent(double n);
 void launchPowSelfTest(const double* x, int n, double e, double* fast, double* ref);
 void launchStencilSelfTest(const double* x, int n, int scheme, int op, double* out);
+void launchStencilGroupSelfTest(const double* x, int n, int scheme, int form, double* out);
 Tile makeTile(const DevBlock& b, int tx, int ty, int tz);
 
 }  // namespace mgd

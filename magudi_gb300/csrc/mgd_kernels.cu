@@ -2699,9 +2699,39 @@ __global__ void kStencilSelfTest(const double* __restrict__ x, int n, int scheme
                      : fixedReciprocal(c[0]);
 }
 
+// The stencils that the stage kernels form together: form 0 the first
+// derivative of three fields, 1 its adjoint of four (n groups of windows), 2
+// and 3 the composite dissipation over two and three axes (n boxes of 9^2 or
+// 9^3 points, at the centre).
+__global__ void kStencilGroupSelfTest(const double* __restrict__ x, int n, int scheme, int form,
+                                      double* __restrict__ out) {
+  const int i = blockIdx.x * kBlock + threadIdx.x;
+  if (i >= n) return;
+  const Axis ax[3] = {{9, 1, 1, scheme}, {9, 1, 9, scheme}, {9, 1, 81, scheme}};
+  const int idx[3] = {4, 4, 4};
+  const long long off[4] = {0, 9, 18, 27};
+  double r[4];
+  if (form == 0) {
+    applyOpFields<OP_D1, 3, true>(x + 27LL * i + 4, off, 4, ax[0], r);
+    for (int k = 0; k < 3; ++k) out[3LL * i + k] = r[k];
+  } else if (form == 1) {
+    applyOpFields<OP_D1ADJ, 4, true>(x + 36LL * i + 4, off, 4, ax[0], r);
+    for (int k = 0; k < 4; ++k) out[4LL * i + k] = r[k];
+  } else if (form == 2) {
+    out[i] = compositeDissipationSum<2, true, 1>(x + 81LL * i + 40, idx, ax);
+  } else {
+    out[i] = compositeDissipationSum<3, true, 1>(x + 729LL * i + 364, idx, ax);
+  }
+}
+
 void launchStencilSelfTest(const double* x, int n, int scheme, int op, double* out) {
   uploadOperatorTables();
   kStencilSelfTest<<<(n + kBlock - 1) / kBlock, kBlock>>>(x, n, scheme, op, out);
+}
+
+void launchStencilGroupSelfTest(const double* x, int n, int scheme, int form, double* out) {
+  uploadOperatorTables();
+  kStencilGroupSelfTest<<<(n + kBlock - 1) / kBlock, kBlock>>>(x, n, scheme, form, out);
 }
 
 void launchPowSelfTest(const double* x, int n, double e, double* fast, double* ref) {
