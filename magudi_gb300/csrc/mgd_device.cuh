@@ -82,25 +82,48 @@ __device__ __forceinline__ double tap(const double* p) {
 }
 
 // Interior stencil of OP in FP64 over the taps p[j] = x_{j+1}, m[j] =
-// x_{-(j+1)} and the centre x0 (unused by skew operators), left to right.
+// x_{-(j+1)} and the centre x0 (unused by skew operators), left to right;
+// spelled out, so that every kernel that holds it rounds alike.
 template <int OP>
 __device__ __forceinline__ double interiorSumFp64(const double* p, const double* m, double x0, int scheme) {
   using S = OpShape<OP>;
   const double* __restrict__ cin = c_ops.interior[scheme][OP];
-  double s = cin[S::half + 1] * (S::skew ? p[0] - m[0] : p[0] + m[0]);
+  double s = __dmul_rn(cin[S::half + 1], S::skew ? p[0] - m[0] : p[0] + m[0]);
 #pragma unroll
-  for (int j = 2; j <= S::half; ++j) s += cin[S::half + j] * (S::skew ? p[j - 1] - m[j - 1] : p[j - 1] + m[j - 1]);
-  return S::skew ? s : s + cin[S::half] * x0;
+  for (int j = 2; j <= S::half; ++j)
+    s = fma(cin[S::half + j], S::skew ? p[j - 1] - m[j - 1] : p[j - 1] + m[j - 1], s);
+  return S::skew ? s : fma(cin[S::half], x0, s);
 }
 
-// Interior stencils of OP of K fields: the first derivatives in integers where
-// the taps allow it.
-template <int OP, int K>
-__device__ __forceinline__ void interiorSums(const double (*p)[4], const double (*m)[4], int scheme, double* out) {
-  static_assert(OP == OP_D1 || OP == OP_D1ADJ, "skew operators");
-  if (c_ops.fixed[scheme][OP].valid && fixedSkew<K>(p, m, c_ops.fixed[scheme][OP], out)) return;
+// The interior taps of point i again, for the rare sums in FP64: volatile
+// loads, so that the taps of the integer sum need not be kept for them.
+__device__ __forceinline__ void interiorTapsAgain(const double* __restrict__ c, int i, long long st, const Axis& ax,
+                                                  double* p, double* m) {
+  const double* line = c - i * st;
 #pragma unroll
-  for (int k = 0; k < K; ++k) out[k] = interiorSumFp64<OP>(p[k], m[k], 0.0, scheme);
+  for (int j = 1; j <= 4; ++j) {
+    p[j - 1] = *(const volatile double*)(line + (long long)wrapIndex(i + j, ax.n, ax.per) * st);
+    m[j - 1] = *(const volatile double*)(line + (long long)wrapIndex(i - j, ax.n, ax.per) * st);
+  }
+}
+
+// Interior stencils of OP of K fields, c + off(k): the first derivatives in
+// integers where the taps allow it, field by field.
+template <int OP, int K, class Off>
+__device__ __forceinline__ void interiorSums(const double (*p)[4], const double (*m)[4], const double* __restrict__ c,
+                                             Off off, int i, long long st, const Axis& ax, double* out) {
+  static_assert(OP == OP_D1 || OP == OP_D1ADJ, "skew operators");
+  const FixedOp& F = c_ops.fixed[ax.scheme][OP];
+  unsigned redo = (1u << K) - 1u;
+  if (F.valid) redo = fixedSkew<K>(p, m, F, out);
+  if (redo == 0) return;
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (redo >> k & 1u) {
+      double pk[4], mk[4];
+      interiorTapsAgain(c + off(k), i, st, ax, pk, mk);
+      out[k] = interiorSumFp64<OP>(pk, mk, 0.0, ax.scheme);
+    }
 }
 
 // Boundary closure row of point i (i < depth or i >= n - depth) of a
@@ -181,7 +204,7 @@ __device__ __forceinline__ double applyOp(const double* __restrict__ c, int i, c
   }
   if constexpr (OP == OP_D1 || OP == OP_D1ADJ) {
     double s;
-    interiorSums<OP, 1>(&p, &m, ax.scheme, &s);
+    interiorSums<OP, 1>(&p, &m, c, [](int) { return 0LL; }, i, st, ax, &s);
     return s;
   } else {
     return interiorSumFp64<OP>(p, m, S::skew ? 0.0 : tap<NC>(c), ax.scheme);
@@ -217,7 +240,7 @@ __device__ __forceinline__ void applyOpFields(const double* __restrict__ c, cons
   double p[K][4], m[K][4];
 #pragma unroll
   for (int k = 0; k < K; ++k) interiorTaps<4, NC>(c + off[k], i, st, ax, p[k], m[k]);
-  interiorSums<OP, K>(p, m, ax.scheme, out);
+  interiorSums<OP, K>(p, m, c, [&](int k) { return off[k]; }, i, st, ax, out);
 }
 
 // The composite dissipation's interior stencils of nAxes axes summed, in

@@ -139,45 +139,42 @@ __device__ __forceinline__ double skewFixed(const double* p, const double* m, ui
   return packFixed<false>(T, (uint32_t)lo, E, F);
 }
 
-// K skew stencils at once: false when one of them needs FP64. A field at rest
-// (all taps zero) is in range. One branch for all K leaves their sums in one
-// block of code, which the compiler interleaves.
+// K skew stencils at once; the bits of the fields that need the FP64 sum (a
+// field's result does not depend on the others'). A field at rest (all taps
+// zero) needs none. One branch for all K leaves their sums in one block of
+// code, which the compiler interleaves.
 template <int K>
-__device__ __forceinline__ bool fixedSkew(const double (*p)[4], const double (*m)[4], const FixedOp& F, double* out) {
+__device__ __forceinline__ unsigned fixedSkew(const double (*p)[4], const double (*m)[4], const FixedOp& F,
+                                              double* out) {
   if constexpr (K == 1) {
     // no value live across the branch
     const uint32_t t = largestTap(p[0], m[0]);
     if (!inFixedRange(t)) {
       out[0] = 0.0;
-      return allZero(p[0], 4) && allZero(m[0], 4);
+      return allZero(p[0], 4) && allZero(m[0], 4) ? 0u : 1u;
     }
     out[0] = skewFixed(p[0], m[0], t, F);
-    return true;
+    return 0u;
   }
   uint32_t top[K];
-  bool zero[K], ok = true;
+  unsigned zero = 0, redo = 0;
+  bool ok = true;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     top[k] = largestTap(p[k], m[k]);
-    zero[k] = false;
     ok = ok && inFixedRange(top[k]);
   }
   if (!ok) {
-    ok = true;
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      if (!inFixedRange(top[k])) {
-        zero[k] = allZero(p[k], 4) && allZero(m[k], 4);
-        ok = ok && zero[k];
-      }
-    if (!ok) return false;
+      if (!inFixedRange(top[k])) (allZero(p[k], 4) && allZero(m[k], 4) ? zero : redo) |= 1u << k;
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const double s = skewFixed(p[k], m[k], top[k], F);
-    out[k] = zero[k] ? 0.0 : s;
+    out[k] = zero >> k & 1u ? 0.0 : s;
   }
-  return true;
+  return redo;
 }
 
 // Symmetric stencils of the nAxes axes through a point summed, x0 the centre
