@@ -110,8 +110,8 @@ __device__ __forceinline__ void interiorTapsAgain(const double* __restrict__ c, 
 // Interior stencils of OP of K fields, c + off(k): the first derivatives in
 // integers where the taps allow it, field by field.
 template <int OP, int K, class Off>
-__device__ __forceinline__ void interiorSums(const double (*p)[4], const double (*m)[4], const double* __restrict__ c,
-                                             Off off, int i, long long st, const Axis& ax, double* out) {
+__device__ __forceinline__ void interiorSums(double (*p)[4], double (*m)[4], const double* __restrict__ c, Off off,
+                                             int i, long long st, const Axis& ax, double* out) {
   static_assert(OP == OP_D1 || OP == OP_D1ADJ, "skew operators");
   const FixedOp& F = c_ops.fixed[ax.scheme][OP];
   unsigned redo = (1u << K) - 1u;
@@ -246,7 +246,7 @@ __device__ __forceinline__ void applyOpFields(const double* __restrict__ c, cons
 // The composite dissipation's interior stencils of nAxes axes summed, in
 // integers where the taps allow it (the taps of the other axes are 0).
 template <int ND>
-__device__ __forceinline__ double compositeInteriorSum(const double (*p)[4], const double (*m)[4], double x0, int nAxes,
+__device__ __forceinline__ double compositeInteriorSum(double (*p)[4], double (*m)[4], double x0, int nAxes,
                                                        int scheme) {
   double s;
   if (c_ops.fixed[scheme][OP_DCOMP].valid && fixedSymmetric<ND>(p, m, x0, nAxes, c_ops.fixed[scheme][OP_DCOMP], s))

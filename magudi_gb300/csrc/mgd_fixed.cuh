@@ -40,6 +40,7 @@ namespace mgd {
 // operator has this form.
 struct FixedOp {
   int a[5];
+  int half;                // taps beyond it have coefficient 0 (padding)
   int shift;
   unsigned flip;           // 0x80000000 when s = -1
   int valid;
@@ -118,6 +119,18 @@ __device__ __forceinline__ uint32_t largestTap(const double* p, const double* m)
 }
 __device__ __forceinline__ bool inFixedRange(uint32_t top) { return (top >> 21) - 128u < 1900u; }
 
+// Finite taps beyond a narrow stencil's half width, whose coefficients are 0,
+// give way to its nearest ones, so that they do not set the unit. Infinities
+// and NaN stay and take the FP64 sum.
+__device__ __forceinline__ void dropPadding(double* p, double* m, int half) {
+#pragma unroll
+  for (int j = 1; j < 4; ++j)
+    if (j >= half) {
+      if ((hiWord(p[j]) & 0x7ff00000u) != 0x7ff00000u) p[j] = p[0];
+      if ((hiWord(m[j]) & 0x7ff00000u) != 0x7ff00000u) m[j] = m[0];
+    }
+}
+
 // Skew stencil over the taps p[j] = x_{j+1}, m[j] = x_{-(j+1)}, whose largest
 // is in range.
 __device__ __forceinline__ double skewFixed(const double* p, const double* m, uint32_t top, const FixedOp& F) {
@@ -144,8 +157,10 @@ __device__ __forceinline__ double skewFixed(const double* p, const double* m, ui
 // zero) needs none. One branch for all K leaves their sums in one block of
 // code, which the compiler interleaves.
 template <int K>
-__device__ __forceinline__ unsigned fixedSkew(const double (*p)[4], const double (*m)[4], const FixedOp& F,
-                                              double* out) {
+__device__ __forceinline__ unsigned fixedSkew(double (*p)[4], double (*m)[4], const FixedOp& F, double* out) {
+  if (F.half < 4)
+#pragma unroll
+    for (int k = 0; k < K; ++k) dropPadding(p[k], m[k], F.half);
   if constexpr (K == 1) {
     // no value live across the branch
     const uint32_t t = largestTap(p[0], m[0]);
@@ -180,8 +195,11 @@ __device__ __forceinline__ unsigned fixedSkew(const double (*p)[4], const double
 // Symmetric stencils of the nAxes axes through a point summed, x0 the centre
 // tap of each (denominator a power of two); the taps of the other axes are 0.
 template <int ND>
-__device__ __forceinline__ bool fixedSymmetric(const double (*p)[4], const double (*m)[4], double x0, int nAxes,
-                                               const FixedOp& F, double& out) {
+__device__ __forceinline__ bool fixedSymmetric(double (*p)[4], double (*m)[4], double x0, int nAxes, const FixedOp& F,
+                                               double& out) {
+  if (F.half < 4)
+#pragma unroll
+    for (int d = 0; d < ND; ++d) dropPadding(p[d], m[d], F.half);
   uint32_t top = hiWord(x0) + hiWord(x0);
 #pragma unroll
   for (int d = 0; d < ND; ++d)

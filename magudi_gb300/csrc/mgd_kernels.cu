@@ -216,6 +216,7 @@ static FixedOp fixedForm(const HostOp& h, int den) {
   for (int j = 0; j <= h.half; ++j) {
     const double c = (j % 2 ? s : -s) * h.I(j) * den;
     f.a[j] = (int)std::lround(c);
+    if (f.a[j]) f.half = j;
     if (f.a[j] < 0 || f.a[j] > 1023 || std::fabs(c - f.a[j]) > 1e-12 || h.I(-j) != (h.skew && j ? -h.I(j) : h.I(j)))
       f.valid = 0;
   }

@@ -1,13 +1,14 @@
 """Interior stencils in integer arithmetic: the forms that take several fields
-at once."""
+or axes at once, and taps that a narrow stencil leaves out."""
 import ctypes as C
+from fractions import Fraction
 
 import numpy as np
 import pytest
 
 from magudi_gb300 import capi
 from magudi_gb300.solver import load_library
-from test_gpu_stencil import KINDS, run, windows
+from test_gpu_stencil import KINDS, coefficients, run, windows
 
 pytestmark = pytest.mark.gpu
 
@@ -21,6 +22,22 @@ def run_groups(x, n, scheme, form):
     out = np.zeros(n * FIELDS.get(form, 1))
     assert L.mgd_selftest_stencil_group(capi.dptr(np.ascontiguousarray(x)), n, scheme, form, capi.dptr(out)) == 0
     return out
+
+
+def rational(c, den, w):
+    return sum(Fraction(v) * Fraction(float(t)) for v, t in zip(c, w)) / den
+
+
+def boxes(axes):
+    """Boxes of 9 points along every axis (x fastest) whose axes through the
+    centre hold the given windows (n, nD, 9); the other points are NaN."""
+    n, nD, _ = axes.shape
+    box = np.full((n,) + (9,) * nD, np.nan)
+    for d in range(nD):
+        line = [slice(None)] + [4] * nD
+        line[nD - d] = slice(None)
+        box[tuple(line)] = axes[:, d]
+    return box.reshape(n, -1)
 
 
 @pytest.mark.parametrize("scheme", SCHEMES)
@@ -43,3 +60,51 @@ def test_fields_together_are_bitwise_the_fields_alone(scheme, form):
     alone = run(x.reshape(-1, 9), scheme, form)
     together = run_groups(x, len(x), scheme, form)
     assert np.array_equal(together.view(np.int64), alone.view(np.int64))
+
+
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("nD", [2, 3])
+def test_dissipation_over_the_axes_against_rational_sums(scheme, nD):
+    """Each tap off by less than one unit, 2^-61 of the largest tap, and one
+    rounding (half up, from 64 bits kept); below the integers' range 16
+    roundings of the products of nine taps per axis and 16 subnormal units."""
+    c, den = coefficients(scheme, 2)
+    total = nD * Fraction(sum(abs(v) for v in c), den)
+    real = [j for j in range(9) if c[j]]
+    for kind in KINDS:
+        axes = windows(kind, 101 * nD, np.random.default_rng(5)).reshape(101, nD, 9).copy()
+        axes[:, :, 4] = axes[:, :1, 4]
+        got = run_groups(boxes(axes), len(axes), scheme, nD)
+        for w, g in zip(axes, got):
+            exact = sum(rational(c, den, a) for a in w)
+            top = Fraction(float(np.abs(w[:, real]).max()))
+            if kind in ("below the integer range", "subnormal"):
+                bound = 16 * nD * total * top / 2 ** 53 + 16 * Fraction(1, 2 ** 1074)
+            else:
+                bound = abs(exact) * (1 + Fraction(1, 256)) / 2 ** 53 + total * top / 2 ** 61
+            assert abs(Fraction(float(g)) - exact) <= bound, (kind, w, g, float(exact))
+
+
+@pytest.mark.parametrize("scheme", SCHEMES[1:])
+@pytest.mark.parametrize("op", [0, 1, 2])
+def test_taps_outside_a_narrow_stencil_do_not_set_its_unit(scheme, op):
+    """The lower-order schemes' stencils are stored in the widest one's shape.
+    Taps that their coefficients leave out may be 2^20 to 2^80 times the
+    others: the sum is as exact as without them."""
+    c, den = coefficients(scheme, op)
+    total = Fraction(sum(abs(v) for v in c), den)
+    real = np.array([v != 0 for v in c]) | (np.arange(9) == 4)
+    rng = np.random.default_rng(7)
+    x = rng.uniform(-1, 1, (400, 9))
+    x[:, ~real] *= 2.0 ** rng.uniform(20, 80, (400, 1))
+    x[200:, real] *= np.where(rng.random((200, int(real.sum()))) < 0.5, 0.0, -1.0)
+    for w, g in zip(x, run(x, scheme, op)):
+        exact = rational(c, den, w)
+        top = Fraction(float(np.abs(w[real]).max()))
+        bound = abs(exact) * (1 + Fraction(1, 256)) / 2 ** 53 + total * top / 2 ** 61
+        assert abs(Fraction(float(g)) - exact) <= bound, (w, g, float(exact))
+    # an undefined tap shows in the result, stencil or padding
+    x = np.ones((9, 9))
+    x[np.arange(9), np.arange(9)] = np.nan
+    x = np.delete(x, 4, axis=0)
+    assert np.all(np.isnan(run(x, scheme, op)))
