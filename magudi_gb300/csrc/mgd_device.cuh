@@ -97,21 +97,26 @@ __device__ __forceinline__ double interiorSumFp64(const double* p, const double*
 
 // The interior taps of point i again, for the rare sums in FP64: volatile
 // loads, so that the taps of the integer sum need not be kept for them.
-__device__ __forceinline__ void interiorTapsAgain(const double* __restrict__ c, int i, long long st, const Axis& ax,
-                                                  double* p, double* m) {
-  const double* line = c - i * st;
+__device__ __forceinline__ void interiorTapsAgain(const double* c, int i, const Axis& ax, double* p, double* m) {
+  const double* line = c - i * ax.stride;
 #pragma unroll
   for (int j = 1; j <= 4; ++j) {
-    p[j - 1] = *(const volatile double*)(line + (long long)wrapIndex(i + j, ax.n, ax.per) * st);
-    m[j - 1] = *(const volatile double*)(line + (long long)wrapIndex(i - j, ax.n, ax.per) * st);
+    p[j - 1] = *(const volatile double*)(line + (long long)wrapIndex(i + j, ax.n, ax.per) * ax.stride);
+    m[j - 1] = *(const volatile double*)(line + (long long)wrapIndex(i - j, ax.n, ax.per) * ax.stride);
   }
+}
+template <int OP>
+__device__ __noinline__ double interiorSumAgain(const double* c, int i, Axis ax) {
+  double p[4], m[4];
+  interiorTapsAgain(c, i, ax, p, m);
+  return interiorSumFp64<OP>(p, m, 0.0, ax.scheme);
 }
 
 // Interior stencils of OP of K fields, c + off(k): the first derivatives in
 // integers where the taps allow it, field by field.
 template <int OP, int K, class Off>
 __device__ __forceinline__ void interiorSums(double (*p)[4], double (*m)[4], const double* __restrict__ c, Off off,
-                                             int i, long long st, const Axis& ax, double* out) {
+                                             int i, const Axis& ax, double* out) {
   static_assert(OP == OP_D1 || OP == OP_D1ADJ, "skew operators");
   const FixedOp& F = c_ops.fixed[ax.scheme][OP];
   unsigned redo = (1u << K) - 1u;
@@ -119,11 +124,7 @@ __device__ __forceinline__ void interiorSums(double (*p)[4], double (*m)[4], con
   if (redo == 0) return;
 #pragma unroll
   for (int k = 0; k < K; ++k)
-    if (redo >> k & 1u) {
-      double pk[4], mk[4];
-      interiorTapsAgain(c + off(k), i, st, ax, pk, mk);
-      out[k] = interiorSumFp64<OP>(pk, mk, 0.0, ax.scheme);
-    }
+    if (redo >> k & 1u) out[k] = interiorSumAgain<OP>(c + off(k), i, ax);
 }
 
 // Boundary closure row of point i (i < depth or i >= n - depth) of a
@@ -204,7 +205,7 @@ __device__ __forceinline__ double applyOp(const double* __restrict__ c, int i, c
   }
   if constexpr (OP == OP_D1 || OP == OP_D1ADJ) {
     double s;
-    interiorSums<OP, 1>(&p, &m, c, [](int) { return 0LL; }, i, st, ax, &s);
+    interiorSums<OP, 1>(&p, &m, c, [](int) { return 0LL; }, i, ax, &s);
     return s;
   } else {
     return interiorSumFp64<OP>(p, m, S::skew ? 0.0 : tap<NC>(c), ax.scheme);
@@ -240,23 +241,24 @@ __device__ __forceinline__ void applyOpFields(const double* __restrict__ c, cons
   double p[K][4], m[K][4];
 #pragma unroll
   for (int k = 0; k < K; ++k) interiorTaps<4, NC>(c + off[k], i, st, ax, p[k], m[k]);
-  interiorSums<OP, K>(p, m, c, [&](int k) { return off[k]; }, i, st, ax, out);
+  interiorSums<OP, K>(p, m, c, [&](int k) { return off[k]; }, i, ax, out);
 }
 
-// The composite dissipation's interior stencils of nAxes axes summed, in
-// integers where the taps allow it (the taps of the other axes are 0).
+// The composite dissipation's interior stencils of the axes summed, in
+// integers where the taps allow it; closed: bits of the axes left out, whose
+// taps are 0.
 template <int ND>
-__device__ __forceinline__ double compositeInteriorSum(double (*p)[4], double (*m)[4], double x0, int nAxes,
+__device__ __forceinline__ double compositeInteriorSum(double (*p)[4], double (*m)[4], double x0, unsigned closed,
                                                        int scheme) {
   double s;
-  if (c_ops.fixed[scheme][OP_DCOMP].valid && fixedSymmetric<ND>(p, m, x0, nAxes, c_ops.fixed[scheme][OP_DCOMP], s))
-    return s;
+  const FixedOp& F = c_ops.fixed[scheme][OP_DCOMP];
+  if (F.valid && fixedSymmetric<ND>(p, m, x0, closed, F, s)) return s;
   const double* __restrict__ cin = c_ops.interior[scheme][OP_DCOMP];
-  s = (nAxes * cin[4]) * x0;
+  s = __dmul_rn((ND - __popc(closed)) * cin[4], x0);
 #pragma unroll
   for (int d = 0; d < ND; ++d)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) s += cin[5 + j] * (p[d][j] + m[d][j]);
+    for (int j = 0; j < 4; ++j) s = fma(cin[5 + j], p[d][j] + m[d][j], s);
   return s;
 }
 
@@ -269,7 +271,7 @@ __device__ __forceinline__ double compositeDissipationSum(const double* __restri
                                                           const Axis* ax) {
   double p[ND][4], m[ND][4], closure = 0.0;
   const double x0 = tap<NC>(c);
-  int interior = 0;
+  unsigned closed = 0;
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
     const long long st = d == 0 ? 1 : ax[d].stride;
@@ -277,14 +279,14 @@ __device__ __forceinline__ double compositeDissipationSum(const double* __restri
       closure += closureSum<OP_DCOMP, NC, CU>(c, idx[d], st, ax[d]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) p[d][j] = m[d][j] = 0.0;
+      closed |= 1u << d;
     } else {
       interiorTaps<4, NC>(c, idx[d], st, ax[d], p[d], m[d]);
-      ++interior;
     }
   }
-  if (interior == 0) return closure;
-  const double s = compositeInteriorSum<ND>(p, m, x0, interior, ax[0].scheme);
-  return interior == ND ? s : s + closure;
+  if (closed == (1u << ND) - 1u) return closure;
+  const double s = compositeInteriorSum<ND>(p, m, x0, closed, ax[0].scheme);
+  return closed ? s + closure : s;
 }
 
 // x != 0.0 with integer operations: false for +0 and -0 only, as the

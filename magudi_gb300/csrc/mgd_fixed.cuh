@@ -16,17 +16,24 @@
 //     and rounded once to a double.
 // So the result carries one rounding of its own and at most a few units of
 // 2^-61 of the largest tap, against one rounding per operation in FP64
-// arithmetic. Taps that are infinite or not numbers, and stencils whose
-// largest tap is near the ends of the exponent range, take the FP64 sum.
+// arithmetic. FP64 does better in one case: large opposite taps cancel and the
+// others are so much smaller that the integers lose bits of them. That case,
+// taps that are infinite or not numbers, and stencils whose largest tap is
+// near the ends of the exponent range take the FP64 sum; so zeros stay zeros
+// on a symmetry line, whatever the sign of the field's zeros.
 //
 // Measured over L1-resident data with 16 warps per SM: 572 cycles per warp and
-// sub-partition for the eight-tap FP64 sum, 206 in integers; and the FP64 pipe
-// is left to the pointwise arithmetic, which runs at the same time. Stage
-// kernels, FP64 sums -> integer sums, microseconds a launch: 128^3 periodic,
-// composite dissipation 623 -> 270 (74% of the integer pipe), gradient/flux
-// 681 -> 425, divergence 701 -> 476, adjoint diffusion 404 -> 246; 201^2,
-// 12.3 -> 8.2, 20.5 -> 16.4, 16.4 -> 12.4 and 10.4 -> 8.3. (By this change
-// alone; the kernels' comments have what followed.)
+// sub-partition for the eight-tap FP64 sum, 206 in integers (before the test
+// for cancelling taps); and the FP64 pipe is left to the pointwise arithmetic,
+// which runs at the same time. Stage kernels, FP64 sums -> integer sums,
+// microseconds a launch: 128^3 periodic, composite dissipation 623 -> 270 (74%
+// of the integer pipe), gradient/flux 681 -> 425, divergence 701 -> 476,
+// adjoint diffusion 404 -> 246; 201^2, 12.3 -> 8.2, 20.5 -> 16.4, 16.4 -> 12.4
+// and 10.4 -> 8.3. (By this change alone; the kernels' comments have what
+// followed.) The test for cancelling taps costs 128^3 2% (a forward / adjoint
+// stage's kernels 997 -> 1020 and 1242 -> 1264) and 201^2 nothing: after the
+// sum, with the taps loaded again in a function of its own; keeping them for
+// it cost 128^3 27%, counting every tap's size 15%.
 #pragma once
 
 #include <cstdint>
@@ -106,8 +113,7 @@ __device__ __forceinline__ bool allZero(const double* t, int n) {
   return (any << 1) == 0;
 }
 
-// Twice the largest high word (sign dropped) of the taps, and whether its
-// exponent lies in the range of the integer form.
+// Twice the largest high word (sign dropped) of the taps.
 __device__ __forceinline__ uint32_t largestTap(const double* p, const double* m) {
   uint32_t top = 0;
 #pragma unroll
@@ -117,7 +123,19 @@ __device__ __forceinline__ uint32_t largestTap(const double* p, const double* m)
   }
   return top;
 }
+
+// Whether the largest tap's exponent lies in the range of the integer form.
 __device__ __forceinline__ bool inFixedRange(uint32_t top) { return (top >> 21) - 128u < 1900u; }
+
+// Whether one of the taps p is zero or more than 9 binary places below the
+// largest tap, so that the integers lose bits of it. (top: its exponent filled
+// with ones. Where opposite taps cancel, those of m are as small as their p.)
+__device__ __forceinline__ bool spreadTaps(const double* p, uint32_t top) {
+  uint32_t low = 0xffffffffu;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) low = min(low, hiWord(p[j]) + hiWord(p[j]));
+  return top - low >= 10u << 21;
+}
 
 // Finite taps beyond a narrow stencil's half width, whose coefficients are 0,
 // give way to its nearest ones, so that they do not set the unit. Infinities
@@ -132,14 +150,22 @@ __device__ __forceinline__ void dropPadding(double* p, double* m, int half) {
 }
 
 // Skew stencil over the taps p[j] = x_{j+1}, m[j] = x_{-(j+1)}, whose largest
-// is in range.
-__device__ __forceinline__ double skewFixed(const double* p, const double* m, uint32_t top, const FixedOp& F) {
+// is in range. cancel: the taps are spread and every pair cancels to below
+// 2^-11 of the largest. The FP64 sum's roundings are then below the bits that
+// the integers lose (2^-61 of the largest tap), and it keeps what the small
+// taps give; zeros on a symmetry line among that.
+__device__ __forceinline__ double skewFixed(const double* p, const double* m, uint32_t top, const FixedOp& F,
+                                            bool& cancel) {
   const uint32_t E = top >> 21;
   top |= 0x1fffffu;
+  const bool spread = spreadTaps(p, top);
   const long long d1 = alignTap(p[0], top) - alignTap(m[0], top);
   const long long d2 = alignTap(m[1], top) - alignTap(p[1], top);
   const long long d3 = alignTap(p[2], top) - alignTap(m[2], top);
   const long long d4 = alignTap(m[3], top) - alignTap(p[3], top);
+  // upper words: the leading bit of the largest tap is bit 29 there
+  auto bits = [](long long d) { return (uint32_t)(d >> 32) + (1u << 18); };
+  cancel = spread && (bits(d1) | bits(d2) | bits(d3) | bits(d4)) < 1u << 19;
   unsigned long long lo = (unsigned long long)(uint32_t)d1 * (uint32_t)F.a[1];
   lo += (unsigned long long)(uint32_t)d2 * (uint32_t)F.a[2];
   lo += (unsigned long long)(uint32_t)d3 * (uint32_t)F.a[3];
@@ -161,15 +187,15 @@ __device__ __forceinline__ unsigned fixedSkew(double (*p)[4], double (*m)[4], co
   if (F.half < 4)
 #pragma unroll
     for (int k = 0; k < K; ++k) dropPadding(p[k], m[k], F.half);
+  bool cancel;
   if constexpr (K == 1) {
-    // no value live across the branch
     const uint32_t t = largestTap(p[0], m[0]);
     if (!inFixedRange(t)) {
       out[0] = 0.0;
       return allZero(p[0], 4) && allZero(m[0], 4) ? 0u : 1u;
     }
-    out[0] = skewFixed(p[0], m[0], t, F);
-    return 0u;
+    out[0] = skewFixed(p[0], m[0], t, F, cancel);
+    return cancel ? 1u : 0u;
   }
   uint32_t top[K];
   unsigned zero = 0, redo = 0;
@@ -186,39 +212,51 @@ __device__ __forceinline__ unsigned fixedSkew(double (*p)[4], double (*m)[4], co
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const double s = skewFixed(p[k], m[k], top[k], F);
-    out[k] = zero >> k & 1u ? 0.0 : s;
+    const double s = skewFixed(p[k], m[k], top[k], F, cancel);
+    const bool rest = zero >> k & 1u;
+    out[k] = rest ? 0.0 : s;
+    if (cancel && !rest) redo |= 1u << k;
   }
   return redo;
 }
 
-// Symmetric stencils of the nAxes axes through a point summed, x0 the centre
-// tap of each (denominator a power of two); the taps of the other axes are 0.
+// Symmetric stencils of the axes through a point summed, x0 the centre tap of
+// each (denominator a power of two); closed: bits of the axes that are left
+// out, whose taps are 0. False when the sum needs FP64.
 template <int ND>
-__device__ __forceinline__ bool fixedSymmetric(double (*p)[4], double (*m)[4], double x0, int nAxes, const FixedOp& F,
-                                               double& out) {
+__device__ __forceinline__ bool fixedSymmetric(double (*p)[4], double (*m)[4], double x0, unsigned closed,
+                                               const FixedOp& F, double& out) {
   if (F.half < 4)
 #pragma unroll
     for (int d = 0; d < ND; ++d) dropPadding(p[d], m[d], F.half);
-  uint32_t top = hiWord(x0) + hiWord(x0);
+  const uint32_t h0 = hiWord(x0) + hiWord(x0);
+  uint32_t top = h0;
 #pragma unroll
-  for (int d = 0; d < ND; ++d)
+  for (int d = 0; d < ND; ++d) top = max(top, largestTap(p[d], m[d]));
+  const uint32_t E = top >> 21, limit = (E - 11u) << 21;
+  if (!inFixedRange(top) || h0 < limit) {
+    // out of range; or a centre below 2^-11 of the largest tap, about which
+    // every pair may cancel to that too: as with skew stencils, the FP64 sum
+    // then keeps what the integers lose
+    bool fp64 = true;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t hp = hiWord(p[d][j]), hm = hiWord(m[d][j]);
-      top = max(top, max(hp + hp, hm + hm));
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t h = hiWord(p[d][j] + m[d][j]);
+        fp64 = fp64 && h + h < limit;
+      }
+    if (fp64 || !inFixedRange(top)) {
+      bool zero = allZero(&x0, 1);
+#pragma unroll
+      for (int d = 0; d < ND; ++d) zero = allZero(p[d], 4) && allZero(m[d], 4) && zero;
+      out = 0.0;
+      return zero;
     }
-  const uint32_t E = top >> 21;
-  if (!inFixedRange(top)) {
-    bool zero = allZero(&x0, 1);
-#pragma unroll
-    for (int d = 0; d < ND; ++d) zero = allZero(p[d], 4) && allZero(m[d], 4) && zero;
-    out = 0.0;
-    return zero;
   }
   top |= 0x1fffffu;
   const long long d0 = alignTap(x0, top);
-  const uint32_t a0 = (uint32_t)(F.a[0] * nAxes);
+  const uint32_t a0 = (uint32_t)(F.a[0] * (ND - __popc(closed)));
   unsigned long long lp = 0, ln = (unsigned long long)(uint32_t)d0 * a0;
   long long T = -((long long)(int)(d0 >> 32) * (int)a0);
   // opposite taps of up to three axes: |sums| < 3 * 2^63, so each axis has its own products

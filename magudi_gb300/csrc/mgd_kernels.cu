@@ -961,7 +961,7 @@ __global__ void __launch_bounds__(tmadiss::TX* tmadiss::TY)
       tp[1][j - 1] = yAt(j), tm[1][j - 1] = yAt(-j);
       tp[2][j - 1] = zAt(j), tm[2][j - 1] = zAt(-j);
     }
-    const double s = compositeInteriorSum<3>(tp, tm, c0[q], 3, B.ax[0].scheme);
+    const double s = compositeInteriorSum<3>(tp, tm, c0[q], 0u, B.ax[0].scheme);
     const long long p = (x0 + tx) + (long long)nx * ((y0 + ty) + (long long)ny * (z0 + i));
     B.dq[p + N * comp] = f * s;
   }

@@ -1,5 +1,5 @@
 """Interior stencils in integer arithmetic: the forms that take several fields
-or axes at once, and taps that a narrow stencil leaves out."""
+or axes at once, and taps of very different size."""
 import ctypes as C
 from fractions import Fraction
 
@@ -108,3 +108,48 @@ def test_taps_outside_a_narrow_stencil_do_not_set_its_unit(scheme, op):
     x[np.arange(9), np.arange(9)] = np.nan
     x = np.delete(x, 4, axis=0)
     assert np.all(np.isnan(run(x, scheme, op)))
+
+
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("op", [0, 1, 2])
+def test_large_opposite_taps_that_cancel(scheme, op):
+    """Large opposite taps whose difference (first derivatives) or sum
+    (dissipation) is exactly zero leave what the small ones give. Bound: that
+    of the FP64 sum over pairs, at most 16 roundings of the pairs' products."""
+    c, den = coefficients(scheme, op)
+    rng = np.random.default_rng(9)
+    n = 400
+    x = rng.uniform(-1, 1, (n, 9)) * 2.0 ** -rng.uniform(12, 90, (n, 1))
+    for k in range(n):
+        big = [j for j in range(1, 5) if rng.random() < 0.5] or [1]
+        for j in big:
+            v = rng.uniform(0.5, 2.0) * rng.choice([-1.0, 1.0])
+            x[k, 4 + j], x[k, 4 - j] = v, (-v if op == 2 else v)
+    x[::7, 4] = 0.0
+    for w, g in zip(x, run(x, scheme, op)):
+        exact = rational(c, den, w)
+        f = [Fraction(float(t)) for t in w]
+        pairs = sum(abs(c[4 + j]) * abs(f[4 + j] - f[4 - j] if op < 2 else f[4 + j] + f[4 - j]) for j in range(1, 5))
+        pairs = (pairs + abs(c[4]) * abs(f[4])) / den
+        assert abs(Fraction(float(g)) - exact) <= 16 * pairs / 2 ** 53, (w, g, float(exact))
+
+
+@pytest.mark.parametrize("scheme", SCHEMES)
+def test_mirrored_fields(scheme):
+    """About a point a field is even about, its derivative is 0; about a point
+    it is odd about, its dissipation is 0, along one axis and over several;
+    zeros of either sign beside them change nothing."""
+    rng = np.random.default_rng(13)
+    h = rng.uniform(-1, 1, (200, 4)) * 2.0 ** rng.integers(-12, 3, (200, 4))
+    c = rng.uniform(-1, 1, (200, 1))
+    even = np.concatenate([h[:, ::-1], c, h], axis=1)
+    odd = np.concatenate([-h[:, ::-1], 0.0 * c, h], axis=1)
+    assert np.all(run(even, scheme, 0) == 0.0) and np.all(run(even, scheme, 1) == 0.0)
+    assert np.all(run(odd, scheme, 2) == 0.0)
+    for nD in (2, 3):
+        axes = np.stack([np.roll(odd, k, axis=0) * [1.0, -1.0, 3.0][k] for k in range(nD)], axis=1)
+        axes[:, :, 4] = 0.0
+        assert np.all(run_groups(boxes(axes), len(axes), scheme, nD) == 0.0)
+    signed = np.array([1.0, -0.0, 2.0, -0.0, 0.0, 0.0, 2.0, 0.0, 1.0])
+    w = np.stack([signed, signed[::-1], -signed])
+    assert np.all(run(w, scheme, 0) == 0.0) and np.all(run(w, scheme, 1) == 0.0)
