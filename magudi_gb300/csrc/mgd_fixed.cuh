@@ -30,10 +30,10 @@
 // of the integer pipe), gradient/flux 681 -> 425, divergence 701 -> 476,
 // adjoint diffusion 404 -> 246; 201^2, 12.3 -> 8.2, 20.5 -> 16.4, 16.4 -> 12.4
 // and 10.4 -> 8.3. (By this change alone; the kernels' comments have what
-// followed.) The test for cancelling taps costs 128^3 2% (a forward / adjoint
-// stage's kernels 997 -> 1020 and 1242 -> 1264) and 201^2 nothing: after the
-// sum, with the taps loaded again in a function of its own; keeping them for
-// it cost 128^3 27%, counting every tap's size 15%.
+// followed.) The test for cancelling taps costs a 64^3 gradient 1%, a batch of
+// 2D runs 4% and single 2D runs below 1%: after the sum, with the taps loaded
+// again in a function of its own; keeping them for it cost the 128^3 forward
+// stage 27%, the smallest and largest of all taps 15%.
 #pragma once
 
 #include <cstdint>
@@ -59,16 +59,23 @@ __device__ __forceinline__ uint32_t hiWord(double x) { return (uint32_t)__double
 // The tap x in units of 2^(E - 1023 - 61): its significand with the leading
 // bit at bit 61, shifted right by its distance from the largest exponent.
 // top = (E << 21) | 0x1fffff. Negative taps are one's complements, i.e. one
-// unit lower than their value (opposite taps of equal sign cancel it).
-__device__ __forceinline__ long long alignTap(double x, uint32_t top) {
+// unit lower than their value (opposite taps of equal sign cancel it). The
+// distance joins `below` from bit 21 on.
+__device__ __forceinline__ long long alignTap(double x, uint32_t top, uint32_t& below) {
   const uint32_t h = hiWord(x), l = (uint32_t)__double2loint(x);
-  const uint32_t s = (top - (h + h)) >> 21;
+  const uint32_t t = top - (h + h), s = t >> 21;
+  below |= t;
   const uint32_t m = (uint32_t)((int)h >> 31);
   const uint32_t hi = (__funnelshift_l(l, h, 9) & 0x1fffffffu) ^ (m ^ 0x20000000u);
   const uint32_t lo = (l << 9) ^ m;
   long long r;  // shr clamps shifts beyond 63
   asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"((long long)(((unsigned long long)hi << 32) | lo)), "r"(s));
   return r;
+}
+
+__device__ __forceinline__ long long alignTap(double x, uint32_t top) {
+  uint32_t below = 0;
+  return alignTap(x, top, below);
 }
 
 // (T 2^32 + r) 2^(E - 1023 - 61) / den as a double, rounded once.
@@ -127,16 +134,6 @@ __device__ __forceinline__ uint32_t largestTap(const double* p, const double* m)
 // Whether the largest tap's exponent lies in the range of the integer form.
 __device__ __forceinline__ bool inFixedRange(uint32_t top) { return (top >> 21) - 128u < 1900u; }
 
-// Whether one of the taps p is zero or more than 9 binary places below the
-// largest tap, so that the integers lose bits of it. (top: its exponent filled
-// with ones. Where opposite taps cancel, those of m are as small as their p.)
-__device__ __forceinline__ bool spreadTaps(const double* p, uint32_t top) {
-  uint32_t low = 0xffffffffu;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) low = min(low, hiWord(p[j]) + hiWord(p[j]));
-  return top - low >= 10u << 21;
-}
-
 // Finite taps beyond a narrow stencil's half width, whose coefficients are 0,
 // give way to its nearest ones, so that they do not set the unit. Infinities
 // and NaN stay and take the FP64 sum.
@@ -150,22 +147,24 @@ __device__ __forceinline__ void dropPadding(double* p, double* m, int half) {
 }
 
 // Skew stencil over the taps p[j] = x_{j+1}, m[j] = x_{-(j+1)}, whose largest
-// is in range. cancel: the taps are spread and every pair cancels to below
-// 2^-11 of the largest. The FP64 sum's roundings are then below the bits that
-// the integers lose (2^-61 of the largest tap), and it keeps what the small
-// taps give; zeros on a symmetry line among that.
+// is in range. cancel: the taps are spread (one of p is zero or 8 or more
+// binary places below the largest; 10 lose bits) and every pair cancels to
+// below 2^-11 of the largest, those of m being as small as their p then. The
+// FP64 sum's roundings are below the bits that the integers lose (2^-61 of the
+// largest tap), and it keeps what the small taps give; zeros on a symmetry
+// line among that.
 __device__ __forceinline__ double skewFixed(const double* p, const double* m, uint32_t top, const FixedOp& F,
                                             bool& cancel) {
   const uint32_t E = top >> 21;
   top |= 0x1fffffu;
-  const bool spread = spreadTaps(p, top);
-  const long long d1 = alignTap(p[0], top) - alignTap(m[0], top);
-  const long long d2 = alignTap(m[1], top) - alignTap(p[1], top);
-  const long long d3 = alignTap(p[2], top) - alignTap(m[2], top);
-  const long long d4 = alignTap(m[3], top) - alignTap(p[3], top);
+  uint32_t below = 0;
+  const long long d1 = alignTap(p[0], top, below) - alignTap(m[0], top);
+  const long long d2 = alignTap(m[1], top) - alignTap(p[1], top, below);
+  const long long d3 = alignTap(p[2], top, below) - alignTap(m[2], top);
+  const long long d4 = alignTap(m[3], top) - alignTap(p[3], top, below);
   // upper words: the leading bit of the largest tap is bit 29 there
   auto bits = [](long long d) { return (uint32_t)(d >> 32) + (1u << 18); };
-  cancel = spread && (bits(d1) | bits(d2) | bits(d3) | bits(d4)) < 1u << 19;
+  cancel = below >= 8u << 21 && (bits(d1) | bits(d2) | bits(d3) | bits(d4)) < 1u << 19;
   unsigned long long lo = (unsigned long long)(uint32_t)d1 * (uint32_t)F.a[1];
   lo += (unsigned long long)(uint32_t)d2 * (uint32_t)F.a[2];
   lo += (unsigned long long)(uint32_t)d3 * (uint32_t)F.a[3];
