@@ -295,9 +295,11 @@ __device__ __forceinline__ double packSignificand(unsigned long long Y, int bias
   return __longlong_as_double((long long)r);
 }
 
-// 1/x: a 32-bit seed Y0 of 1/m from the FP32 reciprocal, e0 = 1 - m Y0 (below
-// 2^-21), and Y0 (1 + e0 + e0^2), whose next term is below 2^-63. Rounded once
-// from 62 bits. Values whose reciprocal is not normal take the division.
+// 1/x, rounded to nearest: a 32-bit seed Y0 of 1/m from the FP32 reciprocal,
+// e0 = 1 - m Y0 (below 2^-21), and Y0 (1 + e0 + e0^2), whose next term is below
+// 2^-63, rounded to 53 bits Q; its residual 2^105 - Q M, exact in 64 bits, then
+// tells whether a neighbour is nearer (it is for one in a thousand, never by
+// more than one unit). Values whose reciprocal is not normal take the division.
 __device__ __forceinline__ double fixedReciprocal(double x) {
   const uint32_t h = hiWord(x), l = (uint32_t)__double2loint(x);
   const int be = (int)((h >> 20) & 0x7ffu);
@@ -315,7 +317,11 @@ __device__ __forceinline__ double fixedReciprocal(double x) {
   const long long c = e0 + (((long long)eh * eh) >> 27);      // Q75
   const unsigned long long Y =
       ((unsigned long long)y0 << 32) + (unsigned long long)(__mul64hi((long long)y0 << 31, c) >> 10) - 2;  // Q64
-  const double r = packSignificand(Y, 2045 - be);
+  const long long M53 = (long long)(M >> 11);
+  long long Q = (long long)((Y >> 11) + ((Y >> 10) & 1u));
+  const long long R2 = -2 * (long long)((unsigned long long)Q * (unsigned long long)M53);
+  Q += (R2 > M53 ? 1 : 0) - (R2 < -M53 ? 1 : 0);
+  const double r = __longlong_as_double(Q + ((long long)(2044 - be) << 52));
   return __hiloint2double((int)((uint32_t)__double2hiint(r) | (h & 0x80000000u)), __double2loint(r));
 }
 
