@@ -382,6 +382,14 @@ struct DualN {
   }
 };
 __host__ __device__ inline double valueOf(double x) { return x; }
+
+// a / b rounded to nearest from the rounded reciprocal of b: the product's
+// residual is exact (P. Markstein, IBM J. Res. Dev. 34(1), 1990). Three
+// operations where several quotients share a divisor, instead of ten.
+__host__ __device__ inline double quotient(double a, double b, double inv) {
+  const double r = a * inv;
+  return fma(fma(-b, r, a), inv, r);
+}
 template <int K> __host__ __device__ inline double valueOf(const DualN<K>& x) { return x.v; }
 template <int K> __host__ __device__ inline DualN<K> operator+(const DualN<K>& a, const DualN<K>& b) {
   DualN<K> r(a.v + b.v);
@@ -404,9 +412,8 @@ template <int K> __host__ __device__ inline DualN<K> operator*(const DualN<K>& a
   return r;
 }
 template <int K> __host__ __device__ inline DualN<K> operator/(const DualN<K>& a, const DualN<K>& b) {
-  // one FP64 division (about ten instructions) for the value and the derivatives
-  const double inv = 1.0 / b.v;
-  DualN<K> r(a.v * inv);
+  const double inv = 1.0 / b.v;  // about ten instructions
+  DualN<K> r(quotient(a.v, b.v, inv));
   for (int k = 0; k < K; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * inv;
   return r;
 }
@@ -424,10 +431,15 @@ template <int K> __host__ __device__ inline DualN<K> operator*(const DualN<K>& a
   return r;
 }
 template <int K> __host__ __device__ inline DualN<K> operator*(double a, const DualN<K>& b) { return b * a; }
-template <int K> __host__ __device__ inline DualN<K> operator/(const DualN<K>& a, double b) { return a / DualN<K>(b); }
+template <int K> __host__ __device__ inline DualN<K> operator/(const DualN<K>& a, double b) {
+  const double inv = 1.0 / b;
+  DualN<K> r(quotient(a.v, b, inv));
+  for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * inv;
+  return r;
+}
 template <int K> __host__ __device__ inline DualN<K> operator/(double a, const DualN<K>& b) {
   const double inv = 1.0 / b.v;
-  DualN<K> r(a * inv);
+  DualN<K> r(quotient(a, b.v, inv));
   for (int k = 0; k < K; ++k) r.d[k] = -(r.v * b.d[k]) * inv;
   return r;
 }
@@ -445,12 +457,14 @@ template <int K> __host__ __device__ inline DualN<K> sqrtOf(const DualN<K>& a) {
 
 // Roe average of two conserved states (computeRoeAverage,
 // src/CNSHelperImpl.f90:179-351, without the variations). Of dual numbers, the
-// right state may be plain (not differentiated).
+// right state may be plain (not differentiated). Every quotient is rounded
+// once: products with rounded reciprocals made the average's error 5 to 8%
+// larger (random states, against 40 digits).
 template <int ND, class S, class SR>
 __host__ __device__ inline void roeAverage(const S* qL, const SR* qR, double g, S* roe) {
   const S sL = sqrtOf(qL[0]);
   const SR sR = sqrtOf(qR[0]);
-  const S vL = 1.0 / qL[0], w = 1.0 / (sL + sR);
+  const S vL = 1.0 / qL[0], w = sL + sR;
   const SR vR = 1.0 / qR[0];
   S mL2 = qL[1] * qL[1];
   SR mR2 = qR[1] * qR[1];
@@ -461,11 +475,11 @@ __host__ __device__ inline void roeAverage(const S* qL, const SR* qR, double g, 
   const S hL = g * qL[ND + 1] - 0.5 * (g - 1.0) * vL * mL2;
   const SR hR = g * qR[ND + 1] - 0.5 * (g - 1.0) * vR * mR2;
   roe[0] = sL * sR;
-  for (int d = 0; d < ND; ++d) roe[1 + d] = (sR * qL[1 + d] + sL * qR[1 + d]) * w;
-  roe[ND + 1] = (sR * hL + sL * hR) * w;
+  for (int d = 0; d < ND; ++d) roe[1 + d] = (sR * qL[1 + d] + sL * qR[1 + d]) / w;
+  roe[ND + 1] = (sR * hL + sL * hR) / w;
   S m2 = roe[1] * roe[1];
   for (int d = 1; d < ND; ++d) m2 = m2 + roe[1 + d] * roe[1 + d];
-  roe[ND + 1] = (roe[ND + 1] + 0.5 * (g - 1.0) / roe[0] * m2) * (1.0 / g);
+  roe[ND + 1] = (roe[ND + 1] + 0.5 * (g - 1.0) / roe[0] * m2) / g;
 }
 
 // The incoming Jacobian A+ of incomingJacobian below without its matrix. With
@@ -488,7 +502,7 @@ __host__ __device__ inline Incoming<ND, S> incomingState(const S* cv, const doub
   for (int d = 0; d < ND; ++d) arc += metrics[d] * metrics[d];
   arc = sqrt(arc);
   const double arcInv = 1.0 / arc;
-  for (int d = 0; d < ND; ++d) I.n[d] = metrics[d] * arcInv;
+  for (int d = 0; d < ND; ++d) I.n[d] = quotient(metrics[d], arc, arcInv);
   const S v = 1.0 / cv[0];
   for (int d = 0; d < ND; ++d) I.u[d] = v * cv[1 + d];
   S u2 = I.u[0] * I.u[0];
