@@ -550,8 +550,15 @@ int mgd_tune_run(mgd_ctx* ctx, int n_steps, int save_interval, int with_adjoint,
  * 1 dissipation, 2 divergence + RK update, 3 adjoint core, 4 adjoint
  * diffusion, 5 adjoint assembly + RK update. set != 0 gives every block of
  * the context that tile from the next launch on (tile[0..2] >= 1 with a
- * product of at most 256); set = 0 writes the current tile to tile[0..2]. */
+ * product of at most 256); set = 0 writes the current tile to tile[0..2]. The
+ * assembly of viscous 2D blocks has two forms, with and without the diffusion,
+ * with a tile each: both are set, that of the form in use is read. */
 int mgd_stage_tile(mgd_ctx* ctx, int kernel, int* tile, int set);
+
+/* Measurement and test hook (no reference counterpart): the form of the first
+ * block's last adjoint assembly launch, 1 with the diffusion, 0 without, -1
+ * before any; its tile goes to tile[0..2] (tile may be NULL). */
+int mgd_assembly_launch(mgd_ctx* ctx, int* tile);
 
 #ifdef __cplusplus
 }

@@ -251,23 +251,44 @@ int mgd_set_trajectory_storage(mgd_ctx* h, int enable, double max_bytes) {
   return 0;
 }
 
+// The slots of a block's stage-kernel tiles: the six of mgd_stage_tile, the
+// assembly in the form with kernels of its own, and the assembly that forms the
+// diffusion.
+constexpr int kTileSlots = 7;
+static std::array<Tile*, kTileSlots> tileSlots(DevBlock& b) {
+  return {&b.tGrad, &b.tDiss, &b.tRhs, &b.tAdjA, &b.tAdjD, &b.tAdjB, &b.tAdjF};
+}
+// Slot of stage kernel k: of the assembly, that of the form launched last.
+static Tile& tileSlot(Context& c, DevBlock& b, int k) {
+  if (k == 5 && (b.assembleForm < 0 ? assemblyFormsDiffusion(c, b) : b.assembleForm == 1)) return b.tAdjF;
+  return *tileSlots(b)[k];
+}
+
 int mgd_stage_tile(mgd_ctx* h, int kernel, int* tile, int set) {
   Context& c = h->c;
   if (kernel < 0 || kernel > 5 || !tile) return fail(c, "mgd_stage_tile: kernel must be 0..5 and tile non-null");
   if (c.blocks.empty()) return fail(c, "mgd_stage_tile: no blocks");
-  auto slot = [&](DevBlock& b) -> Tile& {
-    Tile* s[6] = {&b.tGrad, &b.tDiss, &b.tRhs, &b.tAdjA, &b.tAdjD, &b.tAdjB};
-    return *s[kernel];
-  };
   if (!set) {
-    const Tile& t = slot(c.blocks[0]);
+    const Tile& t = tileSlot(c, c.blocks[0], kernel);
     for (int d = 0; d < 3; ++d) tile[d] = t.t[d];
     return 0;
   }
   if (tile[0] < 1 || tile[1] < 1 || tile[2] < 1 || (long long)tile[0] * tile[1] * tile[2] > 256)
     return fail(c, "mgd_stage_tile: tile extents must be >= 1 with at most 256 threads");
-  for (auto& b : c.blocks) slot(b) = makeTile(b, tile[0], tile[1], tile[2]);
+  for (auto& b : c.blocks) {
+    *tileSlots(b)[kernel] = makeTile(b, tile[0], tile[1], tile[2]);
+    if (kernel == 5) b.tAdjF = b.tAdjB;  // whichever form a run takes
+  }
   return 0;
+}
+
+int mgd_assembly_launch(mgd_ctx* h, int* tile) {
+  Context& c = h->c;
+  if (c.blocks.empty() || c.blocks[0].assembleTile.t[0] == 0) return -1;  // none yet
+  const DevBlock& b = c.blocks[0];
+  if (tile)
+    for (int d = 0; d < 3; ++d) tile[d] = b.assembleTile.t[d];
+  return b.assembleForm;
 }
 
 int mgd_adjoint_core_lanes(mgd_ctx* h, int lanes) {
@@ -470,7 +491,7 @@ int mgd_add_block(mgd_ctx* h, const mgd_block_desc* desc, const double* coordina
     v.ax[i].scheme = c.opts.discretization_scheme;
   }
   v.curvilinear = c.opts.curvilinear;
-  b.tGrad = b.tDiss = b.tRhs = b.tAdjA = b.tAdjD = b.tAdjB = c.nD == 2 ? makeTile(b, 32, 4, 1) : makeTile(b, 32, 2, 2);
+  for (Tile* t : tileSlots(b)) *t = c.nD == 2 ? makeTile(b, 32, 4, 1) : makeTile(b, 32, 2, 2);
   const long long N = v.N;
   const int nD = c.nD, nU = c.nU;
   PrimLayout L{nD};
@@ -669,12 +690,12 @@ struct TuneKey {
   }
 };
 
-// Tiles of the six stage kernels of a block, shared by all contexts of the
+// Tiles of the stage kernels of a block, shared by all contexts of the
 // process (contexts may be set up from several threads): filled by the
 // per-kernel autotuner at setup and replaced by mgd_tune_run.
 struct Tuned {
-  std::array<Tile, 6> tiles;
-  int gradLanes, coreLanes;
+  std::array<Tile, kTileSlots> tiles;
+  int gradLanes, coreLanes, assembleForm;
 };
 static std::map<TuneKey, Tuned> g_tuneCache;
 static std::mutex g_tuneCacheMutex;
@@ -684,26 +705,36 @@ static TuneKey tuneKey(const Context& c, const DevBlock& b) {
                  c.phys.composite};
 }
 
-static void storeTuned(const Context& c, const DevBlock& b) {
-  const Tile* slots[6] = {&b.tGrad, &b.tDiss, &b.tRhs, &b.tAdjA, &b.tAdjD, &b.tAdjB};
-  Tuned entry;
-  for (int k = 0; k < 6; ++k) entry.tiles[k] = *slots[k];
-  entry.gradLanes = b.gradLanes;
-  entry.coreLanes = b.coreLanes;
+// A block's tiles and forms, and back.
+static Tuned tunedOf(DevBlock& b) {
+  Tuned t;
+  for (int k = 0; k < kTileSlots; ++k) t.tiles[k] = *tileSlots(b)[k];
+  t.gradLanes = b.gradLanes;
+  t.coreLanes = b.coreLanes;
+  t.assembleForm = b.assembleForm;
+  return t;
+}
+static void applyTuned(DevBlock& b, const Tuned& t) {
+  for (int k = 0; k < kTileSlots; ++k) *tileSlots(b)[k] = t.tiles[k];
+  b.gradLanes = t.gradLanes;
+  b.coreLanes = t.coreLanes;
+  b.assembleForm = t.assembleForm;
+}
+
+static void storeTuned(const Context& c, DevBlock& b) {
+  const Tuned entry = tunedOf(b);
   std::lock_guard<std::mutex> lock(g_tuneCacheMutex);
   g_tuneCache[tuneKey(c, b)] = entry;
 }
 
 static int autotune(Context& c, DevBlock& b) {
   const TuneKey key = tuneKey(c, b);
-  Tile* slots[6] = {&b.tGrad, &b.tDiss, &b.tRhs, &b.tAdjA, &b.tAdjD, &b.tAdjB};
+  const auto slots = tileSlots(b);
   {
     std::lock_guard<std::mutex> lock(g_tuneCacheMutex);
     auto it = g_tuneCache.find(key);
     if (it != g_tuneCache.end()) {
-      for (int k = 0; k < 6; ++k) *slots[k] = it->second.tiles[k];
-      b.gradLanes = it->second.gradLanes;
-      b.coreLanes = it->second.coreLanes;
+      applyTuned(b, it->second);
       return 0;
     }
   }
@@ -744,26 +775,25 @@ static int autotune(Context& c, DevBlock& b) {
     return ms;
   };
   const long long saved = c.launches;
-  for (int k = 0; k < 6; ++k) {
+  for (int k = 0; k < kTileSlots; ++k) {
     if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous)) continue;
+    // the assembly with and without the diffusion, each where some run takes it
+    if (k == 5 && !separateAssemblyRuns(c, b)) continue;
+    if (k == 6 && !assemblyFormsDiffusion(c, b)) continue;
+    c.recomputesBeside = k == 4 || k == 5;  // the separate kernels
     auto launch = [&]() {
       switch (k) {
         case 0: launchGradFlux(c, b, true, false, &rs, 1, false); break;
         case 1: launchDissipation(c, b, b.v.q, 1.0); break;
         case 2: launchForwardDivergence(c, b, 0, rs, true, false, c.nD == 2); break;
         case 3: launchAdjointCore(c, b, rs, 1, false); break;
-        case 4:
-          // the separate kernel, which runs of larger blocks use beside the recomputation
-          c.recomputesBeside = true;
-          launchAdjointDiffusion(c, b);
-          c.recomputesBeside = false;
-          break;
+        case 4: launchAdjointDiffusion(c, b); break;
         default: launchAdjointAssemble(c, b, 0, rs, 1, 0.0, true, false); break;
       }
     };
     // the gradient/flux kernel of 2D blocks also has a two-lanes-per-point form
     const int nLaneForms = (k == 0 && c.nD == 2) ? 2 : 1;
-    const auto& kc = c.nD == 2 && (k == 2 || (k == 5 && assemblyFormsDiffusion(c, b))) ? candsAllComponents2D : cands;
+    const auto& kc = c.nD == 2 && (k == 2 || k == 6) ? candsAllComponents2D : cands;
     const int nc = (int)kc.size();
     std::vector<float> ms((size_t)nLaneForms * nc, 1e30f);
     for (int r = 0; r < 20; ++r) launch();  // clocks up before the first timing
@@ -786,6 +816,9 @@ static int autotune(Context& c, DevBlock& b) {
     *slots[k] = makeTile(b, kc[best % nc][0], kc[best % nc][1], kc[best % nc][2]);
     if (k == 0) b.gradLanes = best / nc + 1;
   }
+  c.recomputesBeside = false;
+  b.assembleForm = -1;
+  b.assembleTile = Tile{};
   c.launches = saved;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -2778,7 +2811,7 @@ int mgd_run_adjoint(mgd_ctx* h, double* sensitivity) {
   rb.v = twoLanes ? c.shadow : b.v;
   rb.exc = b.exc;
   rb.tGrad = b.tGrad; rb.tDiss = b.tDiss; rb.tRhs = b.tRhs; rb.gradLanes = b.gradLanes; rb.coreLanes = b.coreLanes;
-  rb.tAdjA = b.tAdjA; rb.tAdjD = b.tAdjD; rb.tAdjB = b.tAdjB;
+  rb.tAdjA = b.tAdjA; rb.tAdjD = b.tAdjD; rb.tAdjB = b.tAdjB; rb.tAdjF = b.tAdjF;
   const Lanes adjLanes{c.stream, c.side, c.evFork[1], c.evJoin[1]};
   const Lanes recLanes = twoLanes ? Lanes{c.stream2, c.side2, c.evFork[2], c.evJoin[2]}
                                   : Lanes{c.stream, c.side, c.evFork[0], c.evJoin[0]};
@@ -3566,10 +3599,7 @@ int mgd_tune_run(mgd_ctx* h, int n_steps, int save_interval, int with_adjoint, d
   else
     cands = {{8, 4, 2}, {16, 2, 2}, {32, 2, 1}, {8, 8, 2}, {16, 4, 2}, {32, 2, 2}, {32, 4, 1},
              {16, 8, 1}, {8, 4, 4}, {64, 2, 1}, {16, 4, 4}};
-  auto slotOf = [](DevBlock& b, int k) -> Tile& {
-    Tile* s[6] = {&b.tGrad, &b.tDiss, &b.tRhs, &b.tAdjA, &b.tAdjD, &b.tAdjB};
-    return *s[k];
-  };
+  auto slotOf = [&](DevBlock& b, int k) -> Tile& { return tileSlot(c, b, k); };
   auto setAll = [&](int k, const std::array<int, 3>& t, int lanes) {
     for (auto& b : c.blocks) {
       slotOf(b, k) = makeTile(b, t[0], t[1], t[2]);
@@ -3578,26 +3608,15 @@ int mgd_tune_run(mgd_ctx* h, int n_steps, int save_interval, int with_adjoint, d
     }
   };
   // the tiles and forms on entry, put back if a timed run fails
-  struct Entry {
-    std::array<Tile, 6> tiles;
-    int gradLanes, coreLanes;
-  };
-  std::vector<Entry> entry;
-  for (auto& b : c.blocks) {
-    Entry e;
-    for (int k = 0; k < 6; ++k) e.tiles[k] = slotOf(b, k);
-    e.gradLanes = b.gradLanes;
-    e.coreLanes = b.coreLanes;
-    entry.push_back(e);
-  }
+  std::vector<Tuned> entry;
+  for (auto& b : c.blocks) entry.push_back(tunedOf(b));
   int rc = 0;
   double best = 0.0;
   for (int w = 0; w < 2 && !rc; ++w) rc = runOnce(&best);  // warm-up: clocks, graph buffers
   if (!rc) rc = timed(&best);
   for (int pass = 0; pass < 2 && !rc; ++pass)
     for (int k = 0; k < 6 && !rc; ++k) {
-      if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous) || (k >= 3 && !with_adjoint))
-        continue;
+      if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous) || (k >= 3 && !with_adjoint)) continue;
       const Tile& cur = slotOf(c.blocks[0], k);
       std::array<int, 3> bestT = {cur.t[0], cur.t[1], cur.t[2]};
       int bestLanes = k == 3 ? c.blocks[0].coreLanes : c.blocks[0].gradLanes;
@@ -3619,12 +3638,7 @@ int mgd_tune_run(mgd_ctx* h, int n_steps, int save_interval, int with_adjoint, d
     }
   if (rc) {
     const std::string err = c.error;
-    for (size_t i = 0; i < c.blocks.size(); ++i) {
-      DevBlock& b = c.blocks[i];
-      for (int k = 0; k < 6; ++k) slotOf(b, k) = entry[i].tiles[k];
-      b.gradLanes = entry[i].gradLanes;
-      b.coreLanes = entry[i].coreLanes;
-    }
+    for (size_t i = 0; i < c.blocks.size(); ++i) applyTuned(c.blocks[i], entry[i]);
     c.error = err;
   }
   const int rr = restore();

@@ -226,6 +226,9 @@ struct DevBlock {
   std::vector<ExcPatch> exc;
   // tile shapes of the stage kernels, chosen by the autotuner
   Tile tGrad{}, tDiss{}, tRhs{}, tAdjA{}, tAdjD{}, tAdjB{};
+  Tile tAdjF{};          // the assembly that forms the diffusion too (tAdjB: the separate one)
+  int assembleForm = -1;  // form of the last assembly launch: 1 with the diffusion, 0 separate, -1 none yet
+  Tile assembleTile{};    // its tile
   int gradLanes = 1;  // 2D: kGradFlux with one lane per point (1) or two, one per direction (2)
   int coreLanes = 1;  // 2D: kAdjointCore (1) or kAdjointCoreSplit, one thread per point and direction (2)
   std::vector<void*> allocations;
@@ -497,6 +500,7 @@ void launchExcitation(Context& c, DevBlock& b, const RunScalars& rs, int stage, 
 void launchAdjointSatVectors(Context& c, DevBlock& b, const RunScalars& rs, int stage, bool fromSlot,
                              cudaStream_t s = 0);
 bool assemblyFormsDiffusion(const Context& c, const DevBlock& b);
+bool separateAssemblyRuns(const Context& c, const DevBlock& b);
 void launchAdjointDiffusion(Context& c, DevBlock& b, cudaStream_t s = 0);
 // Adjoint: final assembly, SATs, cost-target forcing and the RK4 adjoint update.
 void launchAdjointAssemble(Context& c, DevBlock& b, int rkStage, const RunScalars& rs, int stage, double apiFactor,

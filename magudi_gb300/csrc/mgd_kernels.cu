@@ -2956,10 +2956,18 @@ void launchAdjointSatVectors(Context& c, DevBlock& b, const RunScalars& rs, int 
 // chain pays while the stage leaves the GPU idle: microseconds per adjoint
 // stage of a resident run, separate / fused, 27.3 / 25.0 at 97x81, 50.7 / 42.7
 // at 201^2, 62.2 / 60.0 at 301x261, 72.8 / 74.1 at 361x301. Beside the
-// recomputation lane, which fills that idle time, only the smallest grids
-// gain: 33.4 / 31.8 at 97x81, 56.1 / 57.8 at 201^2, 87.7 / 88.1 at 301x261.
+// recomputation lane, which fills that idle time, small grids gain: 31.1 / 29.1
+// at 65^2, 32.8 / 31.2 at 97x81, 36.9 / 35.9 at 113^2, 38.2 / 37.6 at 127x129
+// (16,383 points); 151x113 (17,063) loses, 39.8 / 40.6. Beyond, it depends on
+// how the tiles fill the last wave: 46.9 / 44.9 at 151^2, 46.7 / 46.5 at 171^2,
+// 49.0 / 47.6 at 201x161, but 55.1 / 56.1 at 201^2 and 87.7 / 88.1 at 301x261.
+constexpr long long kFusedAssemblyMost = 81920, kFusedAssemblyMostBeside = 16384;
 bool assemblyFormsDiffusion(const Context& c, const DevBlock& b) {
-  return c.nD == 2 && c.phys.viscous && b.v.N <= (c.recomputesBeside ? 16384 : 81920);
+  return c.nD == 2 && c.phys.viscous && b.v.N <= (c.recomputesBeside ? kFusedAssemblyMostBeside : kFusedAssemblyMost);
+}
+// Whether some run of the block launches the separate kernels.
+bool separateAssemblyRuns(const Context& c, const DevBlock& b) {
+  return c.nD != 2 || !c.phys.viscous || b.v.N > kFusedAssemblyMostBeside;
 }
 
 void launchAdjointDiffusion(Context& c, DevBlock& b, cudaStream_t s) {
@@ -2975,14 +2983,13 @@ void launchAdjointAssemble(Context& c, DevBlock& b, int rkStage, const RunScalar
                            bool api, bool fromSlot, cudaStream_t s) {
   cudaStream_t st = on(c, s);
   MGD_LAUNCH(c);
-  if (assemblyFormsDiffusion(c, b)) {
-    const Tile T = b.tAdjB;
-    pdl(kAdjointAssembleDiffusion, T.blocks(), c.nU * T.threads(), st, b.v, c.phys, rs, rkStage, stage, apiFactor, api, fromSlot,
-        T);
+  b.assembleForm = assemblyFormsDiffusion(c, b) ? 1 : 0;
+  const Tile T = b.assembleTile = b.assembleForm == 1 ? b.tAdjF : b.tAdjB;
+  if (b.assembleForm == 1) {
+    pdl(kAdjointAssembleDiffusion, T.blocks(), c.nU * T.threads(), st, b.v, c.phys, rs, rkStage, stage, apiFactor, api,
+        fromSlot, T);
     return;
   }
-  // the fused form's small tile leaves the separate kernel too few threads a CTA
-  const Tile T = c.nD == 2 && c.phys.viscous && b.tAdjB.threads() < 128 ? b.tAdjD : b.tAdjB;
   const dim3 grid(T.blocks(), assemblePerPoint(c.nD) ? 1 : c.nU);
   const int W = T.threads();
 #define AA(ND, VI) \

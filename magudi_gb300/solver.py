@@ -93,6 +93,8 @@ def load_library(build_if_missing=True):
     L.mgd_tune_run.argtypes = [ctx, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double)]
     L.mgd_stage_tile.restype = C.c_int
     L.mgd_stage_tile.argtypes = [ctx, C.c_int, C.POINTER(C.c_int), C.c_int]
+    L.mgd_assembly_launch.restype = C.c_int
+    L.mgd_assembly_launch.argtypes = [ctx, C.POINTER(C.c_int)]
     L.mgd_check_solution_limits.argtypes = [ctx, C.POINTER(C.c_int)]
     L.mgd_batch_persistent.restype = C.c_int
     L.mgd_batch_persistent.argtypes = [C.c_void_p, C.c_int]
@@ -345,6 +347,13 @@ class Solver:
         if tile:
             self._check(self.L.mgd_stage_tile(self.h, int(kernel), t, 0))
         return tuple(t)
+
+    def assembly_launch(self):
+        """(form, tile) of the last adjoint assembly launch: form 1 with the
+        diffusion, 0 without; None before any."""
+        t = (C.c_int * 3)()
+        form = self.L.mgd_assembly_launch(self.h, t)
+        return None if form < 0 else (form, tuple(t))
 
     def dissipation_tma(self, mode=-1):
         """Composite dissipation of fully periodic 3D blocks staged by the
