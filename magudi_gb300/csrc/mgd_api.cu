@@ -778,7 +778,7 @@ static int autotune(Context& c, DevBlock& b) {
   for (int k = 0; k < kTileSlots; ++k) {
     if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous)) continue;
     // the assembly with and without the diffusion, each where some run takes it
-    if (k == 5 && !separateAssemblyRuns(c, b)) continue;
+    if ((k == 4 || k == 5) && !separateAssemblyRuns(c, b)) continue;
     if (k == 6 && !assemblyFormsDiffusion(c, b)) continue;
     c.recomputesBeside = k == 4 || k == 5;  // the separate kernels
     auto launch = [&]() {
@@ -3617,6 +3617,9 @@ int mgd_tune_run(mgd_ctx* h, int n_steps, int save_interval, int with_adjoint, d
   for (int pass = 0; pass < 2 && !rc; ++pass)
     for (int k = 0; k < 6 && !rc; ++k) {
       if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous) || (k >= 3 && !with_adjoint)) continue;
+      // no diffusion kernel in these runs: part of every block's assembly
+      if (k == 4 && std::all_of(c.blocks.begin(), c.blocks.end(), [](const DevBlock& b) { return b.assembleForm == 1; }))
+        continue;
       const Tile& cur = slotOf(c.blocks[0], k);
       std::array<int, 3> bestT = {cur.t[0], cur.t[1], cur.t[2]};
       int bestLanes = k == 3 ? c.blocks[0].coreLanes : c.blocks[0].gradLanes;

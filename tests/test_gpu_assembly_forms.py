@@ -72,3 +72,12 @@ def test_run_level_tuning_keeps_a_tile_it_timed():
     assert s.assembly_launch() == (0, tuned)
     gradient(s, P, True)
     assert s.assembly_launch() == (1, with_diffusion)
+
+
+def test_kernels_that_no_run_launches_are_not_tuned():
+    P = problem(43, 39)
+    s = Solver(P)
+    assert s.assembly_launch() is None
+    assert s.stage_tile(4) == (32, 4, 1)  # the tile before tuning
+    s.tune_run(4, 2)
+    assert s.stage_tile(4) == (32, 4, 1)
