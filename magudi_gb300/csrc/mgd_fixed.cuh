@@ -242,8 +242,9 @@ __device__ __forceinline__ bool fixedSymmetric(double (*p)[4], double (*m)[4], d
     for (int d = 0; d < ND; ++d)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const uint32_t h = hiWord(p[d][j] + m[d][j]);
-        fp64 = fp64 && h + h < limit;
+        // both small, or of opposite sign and alike in 11 places
+        const uint32_t hp = hiWord(p[d][j]), hm = hiWord(m[d][j]) ^ 0x80000000u;
+        fp64 = fp64 && (max(hp + hp, hm + hm) < limit || hp - hm + 510u < 1021u);
       }
     if (fp64 || !inFixedRange(top)) {
       bool zero = allZero(&x0, 1);
