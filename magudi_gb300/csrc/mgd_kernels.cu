@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 #include <utility>
 
@@ -231,7 +232,11 @@ static FixedOp fixedForm(const HostOp& h, int den) {
   return f;
 }
 
+// Contexts may be created from several threads: one fills the (static) host
+// copies and the device's tables at a time.
 void uploadOperatorTables() {
+  static std::mutex mutex;
+  std::lock_guard<std::mutex> lock(mutex);
   static bool done[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
