@@ -743,8 +743,8 @@ __device__ __forceinline__ void gradFluxPoint(const BlockView& B, const Physics&
 }
 
 template <int ND, bool CURV, bool VISC>
-__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).gradFlux) kGradFlux(BlockView B, Physics P, RunScalars rs, int flags,
-                                                      int stage, Tile T) {
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).gradFlux)
+    kGradFlux(BlockView B, Physics P, RunScalars rs, int flags, int stage, Tile T) {
   pdlEnter();
   gradFluxPoint<ND, CURV, VISC>(B, P, rs, flags, stage, T, blockIdx.x);
 }
@@ -785,8 +785,8 @@ __device__ __forceinline__ void dissipationPoint(const BlockView& B, const Physi
 }
 
 template <int ND>
-__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).dissipation) kDissipation(BlockView B, Physics P, const double* __restrict__ src,
-                                                         double sign, Tile T) {
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).dissipation)
+    kDissipation(BlockView B, Physics P, const double* __restrict__ src, double sign, Tile T) {
   pdlEnter();
   dissipationPoint<ND>(B, P, src, sign, T, blockIdx.x);
 }
@@ -1161,9 +1161,9 @@ __device__ __forceinline__ bool forwardDivergencePoint(const BlockView& B, const
 }
 
 template <int ND, bool LIN>
-__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).divergence) kForwardDivergence(BlockView B, Physics P, RunScalars rs, int rkStage,
-                                                               int stage, int controller, Tile T,
-                                                               double linFactor) {
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).divergence)
+    kForwardDivergence(BlockView B, Physics P, RunScalars rs, int rkStage, int stage, int controller, Tile T,
+                       double linFactor) {
   pdlEnter();
   long long p;
   double q;
@@ -1485,8 +1485,8 @@ __global__ void __launch_bounds__(2 * kMaxTile) kAdjointCoreSplit(BlockView B, P
 }
 
 template <int ND, bool CURV, bool VISC>
-__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).core) kAdjointCore(BlockView B, Physics P, RunScalars rs, int stage,
-                                                         int fromSlot, Tile T) {
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).core)
+    kAdjointCore(BlockView B, Physics P, RunScalars rs, int stage, int fromSlot, Tile T) {
   pdlEnter();
   adjointCorePoint<ND, CURV, VISC>(B, P, rs, stage, fromSlot, T, blockIdx.x);
 }
@@ -1824,9 +1824,9 @@ __global__ void __launch_bounds__(kBlock) kExcitation(BlockView B, ExcPatch X, R
 }
 
 template <int ND, bool VISC>
-__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).assemble) kAdjointAssemble(BlockView B, Physics P, RunScalars rs, int rkStage,
-                                                             int stage, double apiFactor, int api, int fromSlot,
-                                                             Tile T) {
+__global__ void __launch_bounds__(kMaxTile, minBlocks(ND).assemble)
+    kAdjointAssemble(BlockView B, Physics P, RunScalars rs, int rkStage, int stage, double apiFactor, int api,
+                     int fromSlot, Tile T) {
   pdlEnter();
   long long p;
   PointIndex I;
