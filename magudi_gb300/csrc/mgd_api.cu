@@ -776,6 +776,7 @@ static int autotune(Context& c, DevBlock& b) {
   };
   const long long saved = c.launches;
   for (int k = 0; k < kTileSlots; ++k) {
+    c.recomputesBeside = false;
     if ((k == 1 && !c.phys.dissipation) || (k == 4 && !c.phys.viscous)) continue;
     // the assembly with and without the diffusion, each where some run takes it
     if ((k == 4 || k == 5) && !separateAssemblyRuns(c, b)) continue;

@@ -60,6 +60,13 @@ def test_a_tile_that_was_set_is_the_one_launched():
             assert s.stage_tile(5) == tile
 
 
+def test_setup_tunes_the_form_with_the_diffusion():
+    """Between the two lines on the number of points both forms run, and both are
+    tuned: at 201x201 compact tiles of 64 points are 10% ahead of the tile before
+    tuning."""
+    assert Solver(problem(201, 201)).stage_tile(5) != (32, 4, 1)
+
+
 def test_run_level_tuning_keeps_a_tile_it_timed():
     """The tile that checkpointed tuning runs leave is that of the kernel they
     launched, and the other form's stays as it was."""
