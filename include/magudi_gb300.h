@@ -452,7 +452,8 @@ int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out
    of three fields (x: n groups of three windows of nine taps, out: 3 n), 1 its
    adjoint of four fields (n groups of four, 4 n), 2 and 3 the composite
    dissipation summed over two and three axes (n boxes of 9^2 or 9^3 points, x
-   fastest, out: its n values at the centres). */
+   fastest, out: its n values at the centres), 4 the first derivative of one
+   field as the persistent batched kernel forms it (n windows, n). */
 int mgd_selftest_stencil_group(const double* x, int n, int scheme, int form, double* out);
 
 /* Self-test of the bounded wait of the persistent batched kernel (no

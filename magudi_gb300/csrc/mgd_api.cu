@@ -3373,8 +3373,8 @@ int mgd_selftest_stencil(const double* x, int n, int scheme, int op, double* out
 }
 
 int mgd_selftest_stencil_group(const double* x, int n, int scheme, int form, double* out) {
-  if (!x || !out || n < 1 || n > (1 << 16) || scheme < 0 || scheme >= kSchemes || form < 0 || form > 3) return 1;
-  static const int in[4] = {3 * 9, 4 * 9, 81, 729}, results[4] = {3, 4, 1, 1};
+  if (!x || !out || n < 1 || n > (1 << 16) || scheme < 0 || scheme >= kSchemes || form < 0 || form > 4) return 1;
+  static const int in[5] = {3 * 9, 4 * 9, 81, 729, 9}, results[5] = {3, 4, 1, 1, 1};
   return selftestOnDevice(x, (size_t)n * in[form], out, (size_t)n * results[form],
                           [&](double* dx, double* dout) { launchStencilGroupSelfTest(dx, n, scheme, form, dout); });
 }

@@ -113,15 +113,23 @@ __device__ __noinline__ double interiorSumAgain(const double* c, int i, Axis ax)
 }
 
 // Interior stencils of OP of K fields, c + off(k): the first derivatives in
-// integers where the taps allow it, field by field.
-template <int OP, int K, class Off>
+// integers where the taps allow it, field by field. The persistent batched
+// kernel (NC = false) has one field at a time and keeps its taps for the FP64
+// sum: a call inside it costs registers in all its phases, 16 runs 21.6 ms
+// against 20.3 without.
+template <int OP, int K, bool NC, class Off>
 __device__ __forceinline__ void interiorSums(double (*p)[4], double (*m)[4], const double* __restrict__ c, Off off,
                                              int i, const Axis& ax, double* out) {
   static_assert(OP == OP_D1 || OP == OP_D1ADJ, "skew operators");
   const FixedOp& F = c_ops.fixed[ax.scheme][OP];
   unsigned redo = (1u << K) - 1u;
-  if (F.valid) redo = fixedSkew<K>(p, m, F, out);
+  if (F.valid) redo = fixedSkew<K, !NC>(p, m, F, out);
   if (redo == 0) return;
+  if constexpr (!NC) {
+    static_assert(K == 1, "one field");
+    out[0] = interiorSumFp64<OP>(p[0], m[0], 0.0, ax.scheme);
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < K; ++k)
     if (redo >> k & 1u) out[k] = interiorSumAgain<OP>(c + off(k), i, ax);
@@ -205,7 +213,7 @@ __device__ __forceinline__ double applyOp(const double* __restrict__ c, int i, c
   }
   if constexpr (OP == OP_D1 || OP == OP_D1ADJ) {
     double s;
-    interiorSums<OP, 1>(&p, &m, c, [](int) { return 0LL; }, i, ax, &s);
+    interiorSums<OP, 1, NC>(&p, &m, c, [](int) { return 0LL; }, i, ax, &s);
     return s;
   } else {
     return interiorSumFp64<OP>(p, m, S::skew ? 0.0 : tap<NC>(c), ax.scheme);
@@ -241,7 +249,7 @@ __device__ __forceinline__ void applyOpFields(const double* __restrict__ c, cons
   double p[K][4], m[K][4];
 #pragma unroll
   for (int k = 0; k < K; ++k) interiorTaps<4, NC>(c + off[k], i, st, ax, p[k], m[k]);
-  interiorSums<OP, K>(p, m, c, [&](int k) { return off[k]; }, i, ax, out);
+  interiorSums<OP, K, NC>(p, m, c, [&](int k) { return off[k]; }, i, ax, out);
 }
 
 // The composite dissipation's interior stencils of the axes summed, in

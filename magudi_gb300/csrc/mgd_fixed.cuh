@@ -30,10 +30,10 @@
 // of the integer pipe), gradient/flux 681 -> 425, divergence 701 -> 476,
 // adjoint diffusion 404 -> 246; 201^2, 12.3 -> 8.2, 20.5 -> 16.4, 16.4 -> 12.4
 // and 10.4 -> 8.3. (By this change alone; the kernels' comments have what
-// followed.) The test for cancelling taps costs a 64^3 gradient 1%, a batch of
-// 2D runs 4% and single 2D runs below 1%: after the sum, with the taps loaded
-// again in a function of its own; keeping them for it cost the 128^3 forward
-// stage 27%, the smallest and largest of all taps 15%.
+// followed.) The test for cancelling taps costs 2D and 3D runs about 1% and the
+// persistent batch 4%: after the sum, with the taps loaded again in a function
+// of its own; keeping them for it cost the 128^3 forward stage 27%, the
+// smallest and largest of all taps 15%.
 #pragma once
 
 #include <cstdint>
@@ -153,6 +153,11 @@ __device__ __forceinline__ void dropPadding(double* p, double* m, int half) {
 // FP64 sum's roundings are below the bits that the integers lose (2^-61 of the
 // largest tap), and it keeps what the small taps give; zeros on a symmetry
 // line among that.
+__device__ __forceinline__ bool pairsCancel(long long d1, long long d2, long long d3, long long d4) {
+  // upper words: the leading bit of the largest tap is bit 29 there
+  auto bits = [](long long d) { return (uint32_t)(d >> 32) + (1u << 18); };
+  return (bits(d1) | bits(d2) | bits(d3) | bits(d4)) < 1u << 19;
+}
 __device__ __forceinline__ double skewFixed(const double* p, const double* m, uint32_t top, const FixedOp& F,
                                             bool& cancel) {
   const uint32_t E = top >> 21;
@@ -162,9 +167,7 @@ __device__ __forceinline__ double skewFixed(const double* p, const double* m, ui
   const long long d2 = alignTap(m[1], top) - alignTap(p[1], top, below);
   const long long d3 = alignTap(p[2], top, below) - alignTap(m[2], top);
   const long long d4 = alignTap(m[3], top) - alignTap(p[3], top, below);
-  // upper words: the leading bit of the largest tap is bit 29 there
-  auto bits = [](long long d) { return (uint32_t)(d >> 32) + (1u << 18); };
-  cancel = below >= 8u << 21 && (bits(d1) | bits(d2) | bits(d3) | bits(d4)) < 1u << 19;
+  cancel = below >= 8u << 21 && pairsCancel(d1, d2, d3, d4);
   unsigned long long lo = (unsigned long long)(uint32_t)d1 * (uint32_t)F.a[1];
   lo += (unsigned long long)(uint32_t)d2 * (uint32_t)F.a[2];
   lo += (unsigned long long)(uint32_t)d3 * (uint32_t)F.a[3];
@@ -177,11 +180,23 @@ __device__ __forceinline__ double skewFixed(const double* p, const double* m, ui
   return packFixed<false>(T, (uint32_t)lo, E, F);
 }
 
+// The same test before the sum, for the kernel that keeps the taps for it.
+__device__ __forceinline__ bool skewCancels(const double* p, const double* m, uint32_t top) {
+  top |= 0x1fffffu;
+  uint32_t below = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) below |= top - (hiWord(p[j]) + hiWord(p[j]));
+  if (below < 8u << 21) return false;
+  return pairsCancel(alignTap(p[0], top) - alignTap(m[0], top), alignTap(m[1], top) - alignTap(p[1], top),
+                     alignTap(p[2], top) - alignTap(m[2], top), alignTap(m[3], top) - alignTap(p[3], top));
+}
+
 // K skew stencils at once; the bits of the fields that need the FP64 sum (a
 // field's result does not depend on the others'). A field at rest (all taps
 // zero) needs none. One branch for all K leaves their sums in one block of
-// code, which the compiler interleaves.
-template <int K>
+// code, which the compiler interleaves. KEEP: decided before the sum, with the
+// taps still at hand.
+template <int K, bool KEEP = false>
 __device__ __forceinline__ unsigned fixedSkew(double (*p)[4], double (*m)[4], const FixedOp& F, double* out) {
   if (F.half < 4)
 #pragma unroll
@@ -189,12 +204,12 @@ __device__ __forceinline__ unsigned fixedSkew(double (*p)[4], double (*m)[4], co
   bool cancel;
   if constexpr (K == 1) {
     const uint32_t t = largestTap(p[0], m[0]);
-    if (!inFixedRange(t)) {
+    if (!inFixedRange(t) || (KEEP && skewCancels(p[0], m[0], t))) {
       out[0] = 0.0;
       return allZero(p[0], 4) && allZero(m[0], 4) ? 0u : 1u;
     }
     out[0] = skewFixed(p[0], m[0], t, F, cancel);
-    return cancel ? 1u : 0u;
+    return !KEEP && cancel ? 1u : 0u;
   }
   uint32_t top[K];
   unsigned zero = 0, redo = 0;

@@ -2710,7 +2710,8 @@ __global__ void kStencilSelfTest(const double* __restrict__ x, int n, int scheme
 // The stencils that the stage kernels form together: form 0 the first
 // derivative of three fields, 1 its adjoint of four (n groups of windows), 2
 // and 3 the composite dissipation over two and three axes (n boxes of 9^2 or
-// 9^3 points, at the centre).
+// 9^3 points, at the centre), 4 the first derivative as the persistent batched
+// kernel forms it (n windows).
 __global__ void kStencilGroupSelfTest(const double* __restrict__ x, int n, int scheme, int form,
                                       double* __restrict__ out) {
   const int i = blockIdx.x * kBlock + threadIdx.x;
@@ -2727,8 +2728,10 @@ __global__ void kStencilGroupSelfTest(const double* __restrict__ x, int n, int s
     for (int k = 0; k < 4; ++k) out[4LL * i + k] = r[k];
   } else if (form == 2) {
     out[i] = compositeDissipationSum<2, true, 1>(x + 81LL * i + 40, idx, ax);
-  } else {
+  } else if (form == 3) {
     out[i] = compositeDissipationSum<3, true, 1>(x + 729LL * i + 364, idx, ax);
+  } else {
+    out[i] = applyOp<OP_D1, false>(x + 9LL * i + 4, 4, ax[0]);
   }
 }
 

@@ -13,7 +13,7 @@ from test_gpu_stencil import KINDS, coefficients, run, windows
 pytestmark = pytest.mark.gpu
 
 SCHEMES = [capi.SBP_48, capi.SBP_12, capi.SBP_24, capi.SBP_36]
-FIELDS = {0: 3, 1: 4}
+FIELDS = {0: 3, 1: 4, 4: 1}
 
 
 def run_groups(x, n, scheme, form):
@@ -41,10 +41,11 @@ def boxes(axes):
 
 
 @pytest.mark.parametrize("scheme", SCHEMES)
-@pytest.mark.parametrize("form", [0, 1])
+@pytest.mark.parametrize("form", [0, 1, 4])
 def test_fields_together_are_bitwise_the_fields_alone(scheme, form):
     """A field's sum does not depend on the other fields': beside ordinary ones
-    some leave the integers' range, are at rest or cancel."""
+    some leave the integers' range, are at rest or cancel. And the persistent
+    batch, which takes one field at a time, forms the same sums."""
     K = FIELDS[form]
     rng = np.random.default_rng(11)
     kinds = KINDS + ["rest", "cancel"]
@@ -57,7 +58,7 @@ def test_fields_together_are_bitwise_the_fields_alone(scheme, form):
                 x[g, k, [2, 6]] = rng.uniform(1, 2)
             elif kind != "rest":
                 x[g, k] = windows(kind, 1, rng)[0]
-    alone = run(x.reshape(-1, 9), scheme, form)
+    alone = run(x.reshape(-1, 9), scheme, form % 4)
     together = run_groups(x, len(x), scheme, form)
     assert np.array_equal(together.view(np.int64), alone.view(np.int64))
 
