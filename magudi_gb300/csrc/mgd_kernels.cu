@@ -89,8 +89,9 @@ __host__ __device__ constexpr bool fieldsTogether(int nD, bool nc) { return nD =
 // CTAs of kMaxTile threads whose registers an SM must hold, per stage kernel.
 // With the stencils in integers the 3D kernels wait for their taps more than
 // for the FP64 pipe, and more warps hide it until the registers spill.
-// Measured at 128^3, microseconds without a bound -> with (the next values in
-// parentheses): gradient/flux 342 at 3 -> 304 at 5 (316 at 4, 298 but 3D jets
+// Measured at 128^3 (before the stencils' test for cancelling taps, with which
+// they take 306, 268, 356, 545, 252 and 199), microseconds without a bound ->
+// with (the next values in parentheses): gradient/flux 342 at 3 -> 304 at 5 (316 at 4, 298 but 3D jets
 // slower at 6), dissipation 270 -> 264 at 4 (281 at 3, 308 at 5), divergence
 // 476 -> 369 at 7 (396 at 6, 369 at 8), core 538 at 3 -> 540 at 4 with jets 6%
 // faster (544 at 5), diffusion 246 -> 242 at 6 (246 at 7), assembly 309 -> 274
@@ -804,9 +805,10 @@ __global__ void __launch_bounds__(kMaxTile, minBlocks(ND).dissipation)
 // another) feed the x and y stencils. Each tap then reads shared memory
 // instead of global memory. The arithmetic is that of dissipationPoint: one
 // integer sum over the taps of all axes (compositeInteriorSum), times
-// sign x amount. Bound by the barrier per plane and the integer pipe: 328 us
-// at 128^3 (631 with FP64 sums) against 260 for kDissipation, 65 against 37
-// at 64^3 and 1077 against 857 at 192^3, so it stays a choice of the caller.
+// sign x amount. Bound by the barrier per plane and the integer pipe: 375
+// to 396 us at 128^3 (631 with FP64 sums) against 268 for kDissipation, 72 to
+// 81 against 39 at 64^3 and 1190 against 900 at 192^3, so it stays a choice of
+// the caller.
 // One elected thread issues the copies; every wait on a copy
 // is bounded, and a wait that runs out sets *err, waits (bounded) for the
 // CTA's copies in flight and leaves.
